@@ -826,8 +826,8 @@ int sht_init(int im, int jm, int km, int nm, double radius, sht_plan **out)
   int lg = 0;
   while ((1 << lg) < im) ++lg;
   const bool pow2 = (1 << lg) == im;
-  // powers of two take the four-step FFT; other even counts (factors 3 and 5,
-  // e.g. 96, 192, 320, 640) the direct transform
+  // powers of two take the four-step FFT; other even counts the mixed-radix
+  // one (factors 3 and 5, e.g. 96, 192, 320, 640) or the direct transform
   if (!zonal && (im < 16 || im > 2048 || (!pow2 && (im & 1)))) {
     set_error("init: im must be 1 (axisymmetric) or even in [16, 2048]");
     return SHT_ERR_UNSUPPORTED_SIZE;

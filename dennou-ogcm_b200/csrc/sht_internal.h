@@ -88,7 +88,7 @@ struct sht_plan_s {
   cudaStream_t copy_in = nullptr, copy_out = nullptr;
   cudaEvent_t chunk_ev[16] = {};
   bool zonal = false;  // im = 1: the axisymmetric (m = 0) transform of wa_zonal_module, lm = nm + 1
-  bool direct_dft = false;  // im not a power of two: longitude transform by direct summation
+  bool direct_dft = false;  // im not a power of two: mixed-radix FFT (factors 2, 3, 5) or, for other prime factors, direct summation
   int M = 0;           // orders transformed: N + 1, or 1 for a zonal plan
   int precision = SHT_PREC_FP64;
   int leg_kernel = 0;  // SHT_OPT_LEGENDRE_KERNEL: 0 auto, 1 per-band, 2 paired persistent, 3 latitude-chunked persistent,
