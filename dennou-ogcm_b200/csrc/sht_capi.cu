@@ -75,9 +75,14 @@ cudaError_t kernel_setup(const void *kern, size_t smem, int threads, int *per_sm
   return cudaSuccess;
 }
 
-// The bounded device-side waits are those of the split-precision kernel; its
-// error word is read only once its tables exist.
-int device_error_status(sht_plan *p) { return split_error_status(p); }
+// The bounded device-side waits are those of the band kernels, whose error
+// word is host memory, and of the split-precision kernel, whose error word is
+// read only once its tables exist.
+int device_error_status(sht_plan *p)
+{
+  const int rc = band_error_status(p);
+  return rc ? rc : split_error_status(p);
+}
 
 namespace {
 
@@ -117,7 +122,8 @@ struct Workspace {
 int ensure_ws(sht_plan *p, int ncol, int nb_temp, Workspace *ws)
 {
   const size_t fbytes = sizeof(double2) * (size_t)(p->N + 1) * ncol * p->J;
-  const size_t sbytes = sizeof(double2) * (size_t)p->R * ncol;
+  // one row more: the synthesis reads the internal rows in pairs
+  const size_t sbytes = sizeof(double2) * (size_t)(p->R + 1) * ncol;
   const size_t wbytes = sizeof(double) * (size_t)p->L * nb_temp;
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
   const size_t need = al(fbytes) + al(sbytes) + al(wbytes);
@@ -616,9 +622,7 @@ int host_call(sht_plan *p, int op, const double *i0, const double *i1, int nb, d
 
 void free_plan(sht_plan *p)
 {
-  cudaFree(p->d_mu); cudaFree(p->d_wgt); cudaFree(p->d_rowscale); cudaFree(p->d_P);
-  cudaFree(p->d_poff); cudaFree(p->d_rowoff); cudaFree(p->d_eps); cudaFree(p->d_tw);
-  cudaFree(p->d_twI); cudaFree(p->d_rn); cudaFree(p->d_spec_tiles); cudaFree(p->d_pairs);
+  cudaFree(p->d_tables);
   cudaFree(p->d_ws); cudaFree(p->d_io);
   if (p->h_stage) cudaFreeHost(p->h_stage);
   free_split_tables(p);

@@ -72,6 +72,15 @@ struct HostGraph {
   int launches = 0;                // kernels in the graph
 };
 
+// A work item of the band kernels: row tiles [t0, t0 + tt) of the output of
+// band m and parity par, whose table starts at block blk, whose coefficients
+// are the cnt internal rows row, row + 2, ...
+struct alignas(16) BandItem {
+  int m, par, t0, tt;
+  long long blk;
+  int row, cnt;
+};
+
 }  // namespace sht
 
 struct sht_plan_s {
@@ -95,7 +104,8 @@ struct sht_plan_s {
                        // 4 single-kernel small-grid transform (plain analysis and synthesis, im <= 128)
   int leg_tile = 0;    // SHT_OPT_LEGENDRE_TILE: 0 auto; paired kernels: analysis columns per item (8, 16); chunked kernels: latitudes per chunk (16, 32)
 
-  // device tables
+  // device tables, all in one allocation
+  void *d_tables = nullptr;
   double *d_mu = nullptr, *d_wgt = nullptr, *d_rowscale = nullptr;
   double *d_P = nullptr;
   long long *d_poff = nullptr;
@@ -111,6 +121,14 @@ struct sht_plan_s {
   int n_pairs = 0;
   int num_sms = 0;
   int sm_cap = 0;       // at most this many SMs' worth of persistent blocks (0: all); set by a batch that runs plans side by side
+
+  // blocked Legendre table and work items of the band kernels (sht_legendre_band.cu)
+  double *d_band_P = nullptr;
+  long long *d_band_off = nullptr;
+  sht::BandItem *d_band_items = nullptr;  // analysis items, then synthesis items
+  int *err_word = nullptr;  // host-mapped word their bounded waits report a timeout in
+  int n_band_f = 0, n_band_i = 0;
+  int band_tf = 0, band_ti = 0;  // most 8-row tiles of an item
 
   // host copies
   std::vector<double> h_mu, h_wgt;
@@ -222,6 +240,13 @@ inline int grid_sms(const sht_plan *p)
 bool leg_pair_supported(const sht_plan *p);
 int launch_leg_fwd_pair(const sht_plan *p, const double2 *F, int ncol, double2 *S, cudaStream_t s);
 int launch_leg_inv_pair(const sht_plan *p, const double2 *S, int ncol, double2 *F, cudaStream_t s);
+
+// --- one band and parity per block, any grid (sht_legendre_band.cu)
+int plan_band_items(sht_plan *p, std::vector<long long> &boff, std::vector<BandItem> &items);
+int build_band_table(sht_plan *p);
+int band_error_status(sht_plan *p);  // reads and clears the plan's error word (after a synchronisation)
+int launch_leg_fwd_band(const sht_plan *p, const double2 *F, int ncol, double2 *S, cudaStream_t s);
+int launch_leg_inv_band(const sht_plan *p, const double2 *S, int ncol, double2 *F, cudaStream_t s);
 
 // --- persistent latitude-chunked FP64 contraction for large grids (sht_legendre_v3.cu)
 bool leg_chunk_supported(const sht_plan *p);

@@ -329,19 +329,15 @@ int launch(K kern, dim3 grid, size_t smem, cudaStream_t s, const LegArgs &args, 
 }  // namespace
 
 // Kernel for the plan's SHT_OPT_LEGENDRE_KERNEL setting: 1 per-band (this
-// file), 2 paired persistent, 3 latitude-chunked persistent; 0 picks the
-// paired kernel where the pair fits in shared memory, else the chunked one,
-// else the per-band one.  A forced choice that does not cover the grid falls
-// back the same way.
+// file), 2 paired persistent, 3 latitude-chunked persistent; otherwise, and
+// where a forced choice does not cover the grid, the band kernels (5).
 int pick_fp64_kernel(const sht_plan *p)
 {
   const int want = p->leg_kernel;
   if (want == 1) return 1;
   if (want == 2 && leg_pair_supported(p)) return 2;
   if (want == 3 && leg_chunk_supported(p)) return 3;
-  if (leg_pair_supported(p)) return 2;
-  if (leg_chunk_supported(p)) return 3;
-  return 1;
+  return 5;
 }
 
 int launch_leg_fwd_fp64(const sht_plan *p, const double2 *F, int ncol, double2 *S, cudaStream_t s)
@@ -350,6 +346,7 @@ int launch_leg_fwd_fp64(const sht_plan *p, const double2 *F, int ncol, double2 *
   switch (pick_fp64_kernel(p)) {
   case 2: return launch_leg_fwd_pair(p, F, ncol, S, s);
   case 3: return launch_leg_fwd_chunk(p, F, ncol, S, s);
+  case 5: return launch_leg_fwd_band(p, F, ncol, S, s);
   default: break;
   }
   LegArgs a{};
@@ -377,6 +374,7 @@ int launch_leg_inv_fp64(const sht_plan *p, const double2 *S, int ncol, double2 *
   switch (pick_fp64_kernel(p)) {
   case 2: return launch_leg_inv_pair(p, S, ncol, F, s);
   case 3: return launch_leg_inv_chunk(p, S, ncol, F, s);
+  case 5: return launch_leg_inv_band(p, S, ncol, F, s);
   default: break;
   }
   LegArgs a{};

@@ -320,7 +320,7 @@ int build(sht_multi *m, int flags)
         wc.push_back(m->inst[i].wa + (long long)k * p->L);
       }
     const size_t fbytes = sizeof(double2) * (size_t)(p->N + 1) * g.ncol * p->J;
-    const size_t sbytes = sizeof(double2) * (size_t)p->R * g.ncol;
+    const size_t sbytes = sizeof(double2) * (size_t)(p->R + 1) * g.ncol;  // the synthesis reads the rows in pairs
     m->groups.push_back(g);
     Group &G = m->groups.back();
     if ((e = cudaMalloc(&G.d_gcol, sizeof(double *) * gc.size())) != cudaSuccess ||

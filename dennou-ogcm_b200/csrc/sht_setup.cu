@@ -10,6 +10,7 @@
 
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 
 namespace sht {
 
@@ -85,13 +86,24 @@ static int ilog2_exact(int n)
   return ((1 << l) == n) ? l : -1;
 }
 
-template <typename T>
-static int dalloc(T **ptr, size_t count)
-{
-  cudaError_t e = cudaMalloc((void **)ptr, sizeof(T) * (count ? count : 1));
-  if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(plan table)");
-  return SHT_OK;
-}
+namespace {
+
+// The plan's tables share one device allocation: parts are reserved first,
+// then the host-built ones are written into one image that goes up in a
+// single copy (a plan had a dozen allocations and uploads, which cost more
+// than its kernels).
+struct TableArena {
+  size_t bytes = 0, host_bytes = 0;
+  template <typename T>
+  size_t reserve(size_t count)
+  {
+    const size_t at = bytes;
+    bytes += (sizeof(T) * (count ? count : 1) + 255) & ~(size_t)255;
+    return at;
+  }
+};
+
+}  // namespace
 
 int build_tables(sht_plan *p)
 {
@@ -102,52 +114,23 @@ int build_tables(sht_plan *p)
   p->R = (long long)(N + 1) * (N + 4) / 2;
   p->M = p->zonal ? 1 : N + 1;
   p->L = p->zonal ? N + 1 : (N + 1) * (N + 1);
-  int rc;
-  // --- Gauss nodes and weights on the device
-  if ((rc = dalloc(&p->d_mu, J)) || (rc = dalloc(&p->d_wgt, J))) return rc;
-  k_gauss_nodes<<<(J / 2 + 127) / 128, 128, 0, p->stream>>>(J, p->d_mu, p->d_wgt);
-  count_launch();
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return cuda_fail(e, "k_gauss_nodes");
-  p->h_mu.resize(J);
-  p->h_wgt.resize(J);
-  if ((e = cudaMemcpyAsync(p->h_mu.data(), p->d_mu, sizeof(double) * J, cudaMemcpyDeviceToHost, p->stream)) != cudaSuccess ||
-      (e = cudaMemcpyAsync(p->h_wgt.data(), p->d_wgt, sizeof(double) * J, cudaMemcpyDeviceToHost, p->stream)) != cudaSuccess ||
-      (e = cudaStreamSynchronize(p->stream)) != cudaSuccess)
-    return cuda_fail(e, "gauss nodes readback");
-
-  // --- recurrence coefficients eps_n^m, n = 0..N+2 (host: closed form)
+  cudaError_t e;
+  // --- host-built tables
+  // recurrence coefficients eps_n^m, n = 0..N+2 (closed form)
   std::vector<double> eps((size_t)(N + 1) * (N + 3));
   for (int m = 0; m <= N; ++m)
     for (int n = 0; n <= N + 2; ++n)
       eps[(size_t)m * (N + 3) + n] = (n < m || n == 0) ? 0.0 : std::sqrt(((double)n * n - (double)m * m) / (4.0 * n * n - 1.0));
-  if ((rc = dalloc(&p->d_eps, eps.size()))) return rc;
-  if ((e = cudaMemcpyAsync(p->d_eps, eps.data(), sizeof(double) * eps.size(), cudaMemcpyHostToDevice, p->stream)) != cudaSuccess)
-    return cuda_fail(e, "eps upload");
-
-  // --- Legendre table on the device
+  // Legendre table and internal row offsets
   std::vector<long long> poff(N + 2);
   long long off = 0;
   for (int m = 0; m <= N; ++m) { poff[m] = off; off += (long long)(N + 2 - m) * JH; }
   poff[N + 1] = off;
-  if ((rc = dalloc(&p->d_poff, N + 2)) || (rc = dalloc(&p->d_P, (size_t)off))) return rc;
-  if ((e = cudaMemcpyAsync(p->d_poff, poff.data(), sizeof(long long) * (N + 2), cudaMemcpyHostToDevice, p->stream)) != cudaSuccess)
-    return cuda_fail(e, "poff upload");
-  dim3 grid((JH + 127) / 128, N + 1);
-  k_legendre_table<<<grid, 128, 0, p->stream>>>(N, J, JH, p->d_mu, p->d_eps, p->d_poff, p->d_P);
-  count_launch();
-  if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "k_legendre_table");
-
-  // --- internal row offsets
   p->h_rowoff.resize(N + 2);
   int ro = 0;
   for (int m = 0; m <= N; ++m) { p->h_rowoff[m] = ro; ro += N + 2 - m; }
   p->h_rowoff[N + 1] = ro;
-  if ((rc = dalloc(&p->d_rowoff, N + 2))) return rc;
-  if ((e = cudaMemcpyAsync(p->d_rowoff, p->h_rowoff.data(), sizeof(int) * (N + 2), cudaMemcpyHostToDevice, p->stream)) != cudaSuccess)
-    return cuda_fail(e, "rowoff upload");
-
-  // --- twiddles (long double on the host, rounded once)
+  // twiddles (long double on the host, rounded once)
   std::vector<double2> tw(NC), twI(NC);
   const long double pi = 3.141592653589793238462643383279502884L;
   for (int k = 0; k < NC; ++k) {
@@ -156,12 +139,64 @@ int build_tables(sht_plan *p)
     long double u = -2.0L * pi * k / I;
     twI[k] = make_double2((double)cosl(u), (double)sinl(u));
   }
-  if ((rc = dalloc(&p->d_tw, NC)) || (rc = dalloc(&p->d_twI, NC))) return rc;
-  if ((e = cudaMemcpyAsync(p->d_tw, tw.data(), sizeof(double2) * NC, cudaMemcpyHostToDevice, p->stream)) != cudaSuccess ||
-      (e = cudaMemcpyAsync(p->d_twI, twI.data(), sizeof(double2) * NC, cudaMemcpyHostToDevice, p->stream)) != cudaSuccess)
-    return cuda_fail(e, "twiddle upload");
+  // Laplacian eigenvalues rn(l,1) = -n(n+1) (zonal layout: l = n)
+  std::vector<double> rn(p->L);
+  for (int n = 0; n <= N; ++n)
+    for (int m = -n; m <= n; ++m)
+      if (!p->zonal) rn[n * (n + 1) + m] = -(double)n * (n + 1);
+      else if (m == 0) rn[n] = -(double)n * (n + 1);
+  // tiles (n, m0) of the spectral layout conversions, n ascending
+  std::vector<int2> tiles;
+  for (int n = 0; n <= N + 1; ++n) {
+    if (n == N + 1) p->n_pack_tiles = (int)tiles.size();
+    const int mmax = p->zonal ? 0 : (n < N ? n : N);
+    for (int m0 = 0; m0 <= mmax; m0 += 32) tiles.push_back(make_int2(n, m0));
+  }
+  p->n_spec_tiles = (int)tiles.size();
+  // band pairs (m, N-m) with N+4 degrees each, plus the middle band of even N
+  std::vector<int2> pairs;
+  if (p->zonal) {
+    pairs.push_back(make_int2(0, -1));  // the m = 0 band alone
+  } else {
+    for (int m = 0; m < N - m; ++m) pairs.push_back(make_int2(m, N - m));
+    if (N % 2 == 0) pairs.push_back(make_int2(N / 2, -1));
+  }
+  p->n_pairs = (int)pairs.size();
+  // items and block offsets of the band kernels
+  std::vector<long long> boff;
+  std::vector<BandItem> items;
+  int rc = plan_band_items(p, boff, items);
+  if (rc) return rc;
 
-  // --- row scales
+  // --- one allocation: the host image's parts, then the device-built tables
+  TableArena ar;
+  const size_t o_eps = ar.reserve<double>(eps.size()), o_poff = ar.reserve<long long>(poff.size());
+  const size_t o_row = ar.reserve<int>(p->h_rowoff.size()), o_tw = ar.reserve<double2>(NC), o_twI = ar.reserve<double2>(NC);
+  const size_t o_rn = ar.reserve<double>(rn.size()), o_tiles = ar.reserve<int2>(tiles.size());
+  const size_t o_pairs = ar.reserve<int2>(pairs.size()), o_boff = ar.reserve<long long>(boff.size());
+  const size_t o_items = ar.reserve<BandItem>(items.size()), o_rs = ar.reserve<double>((size_t)RS_COUNT * J);
+  ar.host_bytes = ar.bytes;
+  const size_t o_mu = ar.reserve<double>(J), o_wgt = ar.reserve<double>(J), o_P = ar.reserve<double>((size_t)off);
+  const size_t o_bP = ar.reserve<double>(64 * (size_t)boff.back());
+  if ((e = cudaMalloc(&p->d_tables, ar.bytes)) != cudaSuccess) return cuda_fail(e, "cudaMalloc(plan tables)");
+  char *const base = static_cast<char *>(p->d_tables);
+  auto at = [&](size_t o, auto *&ptr) { ptr = reinterpret_cast<std::remove_reference_t<decltype(ptr)>>(base + o); };
+  at(o_eps, p->d_eps); at(o_poff, p->d_poff); at(o_row, p->d_rowoff); at(o_tw, p->d_tw); at(o_twI, p->d_twI);
+  at(o_rn, p->d_rn); at(o_tiles, p->d_spec_tiles); at(o_pairs, p->d_pairs); at(o_boff, p->d_band_off);
+  at(o_items, p->d_band_items); at(o_rs, p->d_rowscale); at(o_mu, p->d_mu); at(o_wgt, p->d_wgt); at(o_P, p->d_P);
+  at(o_bP, p->d_band_P);
+
+  // --- Gauss nodes and weights on the device, read back for the row scales
+  k_gauss_nodes<<<(J / 2 + 127) / 128, 128, 0, p->stream>>>(J, p->d_mu, p->d_wgt);
+  count_launch();
+  if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "k_gauss_nodes");
+  p->h_mu.resize(J);
+  p->h_wgt.resize(J);
+  if ((e = cudaMemcpyAsync(p->h_mu.data(), p->d_mu, sizeof(double) * J, cudaMemcpyDeviceToHost, p->stream)) != cudaSuccess ||
+      (e = cudaMemcpyAsync(p->h_wgt.data(), p->d_wgt, sizeof(double) * J, cudaMemcpyDeviceToHost, p->stream)) != cudaSuccess ||
+      (e = cudaStreamSynchronize(p->stream)) != cudaSuccess)
+    return cuda_fail(e, "gauss nodes readback");
+  // row scales
   std::vector<double> rs((size_t)RS_COUNT * J);
   for (int j = 0; j < J; ++j) {
     const double mu = p->h_mu[j], w = p->h_wgt[j];
@@ -174,44 +209,21 @@ int build_tables(sht_plan *p)
     rs[RS_INV_INVACOS * J + j] = 1.0 / (p->radius * c);
     rs[RS_FWD_INVCOS * J + j] = w / (I * c);
   }
-  if ((rc = dalloc(&p->d_rowscale, rs.size()))) return rc;
-  if ((e = cudaMemcpyAsync(p->d_rowscale, rs.data(), sizeof(double) * rs.size(), cudaMemcpyHostToDevice, p->stream)) != cudaSuccess)
-    return cuda_fail(e, "rowscale upload");
+  std::vector<char> image(ar.host_bytes);
+  auto put = [&](size_t o, const auto &v) { std::memcpy(image.data() + o, v.data(), sizeof(v[0]) * v.size()); };
+  put(o_eps, eps); put(o_poff, poff); put(o_row, p->h_rowoff); put(o_tw, tw); put(o_twI, twI); put(o_rn, rn);
+  put(o_tiles, tiles); put(o_pairs, pairs); put(o_boff, boff); put(o_items, items); put(o_rs, rs);
+  if ((e = cudaMemcpyAsync(base, image.data(), ar.host_bytes, cudaMemcpyHostToDevice, p->stream)) != cudaSuccess)
+    return cuda_fail(e, "plan table upload");
 
-  // --- Laplacian eigenvalues rn(l,1) = -n(n+1) (zonal layout: l = n)
-  std::vector<double> rn(p->L);
-  for (int n = 0; n <= N; ++n)
-    for (int m = -n; m <= n; ++m)
-      if (!p->zonal) rn[n * (n + 1) + m] = -(double)n * (n + 1);
-      else if (m == 0) rn[n] = -(double)n * (n + 1);
-  if ((rc = dalloc(&p->d_rn, p->L))) return rc;
-  if ((e = cudaMemcpyAsync(p->d_rn, rn.data(), sizeof(double) * p->L, cudaMemcpyHostToDevice, p->stream)) != cudaSuccess)
-    return cuda_fail(e, "rn upload");
-  // --- tiles (n, m0) of the spectral layout conversions, n ascending
-  std::vector<int2> tiles;
-  for (int n = 0; n <= N + 1; ++n) {
-    if (n == N + 1) p->n_pack_tiles = (int)tiles.size();
-    const int mmax = p->zonal ? 0 : (n < N ? n : N);
-    for (int m0 = 0; m0 <= mmax; m0 += 32) tiles.push_back(make_int2(n, m0));
-  }
-  p->n_spec_tiles = (int)tiles.size();
-  // --- band pairs (m, N-m) with N+4 degrees each, plus the middle band of even N
-  std::vector<int2> pairs;
-  if (p->zonal) {
-    pairs.push_back(make_int2(0, -1));  // the m = 0 band alone
-  } else {
-    for (int m = 0; m < N - m; ++m) pairs.push_back(make_int2(m, N - m));
-    if (N % 2 == 0) pairs.push_back(make_int2(N / 2, -1));
-  }
-  p->n_pairs = (int)pairs.size();
-  if ((rc = dalloc(&p->d_pairs, pairs.size()))) return rc;
-  if ((e = cudaMemcpyAsync(p->d_pairs, pairs.data(), sizeof(int2) * pairs.size(), cudaMemcpyHostToDevice, p->stream)) != cudaSuccess)
-    return cuda_fail(e, "pair table upload");
+  // --- Legendre tables on the device
+  dim3 grid((JH + 127) / 128, N + 1);
+  k_legendre_table<<<grid, 128, 0, p->stream>>>(N, J, JH, p->d_mu, p->d_eps, p->d_poff, p->d_P);
+  count_launch();
+  if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "k_legendre_table");
+  if ((rc = build_band_table(p))) return rc;
   if ((e = cudaDeviceGetAttribute(&p->num_sms, cudaDevAttrMultiProcessorCount, p->device)) != cudaSuccess)
     return cuda_fail(e, "SM count");
-  if ((rc = dalloc(&p->d_spec_tiles, tiles.size()))) return rc;
-  if ((e = cudaMemcpyAsync(p->d_spec_tiles, tiles.data(), sizeof(int2) * tiles.size(), cudaMemcpyHostToDevice, p->stream)) != cudaSuccess)
-    return cuda_fail(e, "spectral tiles upload");
   if ((e = cudaStreamSynchronize(p->stream)) != cudaSuccess) return cuda_fail(e, "plan tables");
   return SHT_OK;
 }
