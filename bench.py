@@ -76,7 +76,9 @@ def _traffic(kernel, mode, nb, grid=GRID):
             t = json.load(f)
     except Exception:
         return None
-    keys = ("k_fft_fwd", "k_fft_inv") if kernel.startswith("k_fft") else ("k_leg_fwd_pair", "k_leg_inv_pair")
+    keys = ("k_fft_fwd", "k_fft_inv") if kernel.startswith("k_fft") else ("k_leg_band_fwd", "k_leg_band_inv")
+    if any(k not in t for k in keys):
+        return None
     return 1e6 * (t[keys[0]] + t[keys[1]]) / 2
 
 

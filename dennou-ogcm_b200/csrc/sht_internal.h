@@ -14,6 +14,7 @@
 //                                 j = JH + jh (JH = J/2), n = m..N+1.
 #pragma once
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <cstdint>
 #include <cstddef>
@@ -100,9 +101,9 @@ struct sht_plan_s {
   bool direct_dft = false;  // im not a power of two: mixed-radix FFT (factors 2, 3, 5) or, for other prime factors, direct summation
   int M = 0;           // orders transformed: N + 1, or 1 for a zonal plan
   int precision = SHT_PREC_FP64;
-  int leg_kernel = 0;  // SHT_OPT_LEGENDRE_KERNEL: 0 auto, 1 per-band, 2 paired persistent, 3 latitude-chunked persistent,
-                       // 4 single-kernel small-grid transform (plain analysis and synthesis, im <= 128)
-  int leg_tile = 0;    // SHT_OPT_LEGENDRE_TILE: 0 auto; paired kernels: analysis columns per item (8, 16); chunked kernels: latitudes per chunk (16, 32)
+  int leg_kernel = 0;  // SHT_OPT_LEGENDRE_KERNEL: 4 single-kernel small-grid transform (plain analysis and synthesis,
+                       // im <= 128); the other values all take the band kernels
+  int leg_tile = 0;    // SHT_OPT_LEGENDRE_TILE: kept for the callers that set it, no kernel has a choice of tiles
 
   // device tables, all in one allocation
   void *d_tables = nullptr;
@@ -129,6 +130,14 @@ struct sht_plan_s {
   int *err_word = nullptr;  // host-mapped word their bounded waits report a timeout in
   int n_band_f = 0, n_band_i = 0;
   int band_tf = 0, band_ti = 0;  // most 8-row tiles of an item
+  // the last data tensor map of each direction: encoding one costs a launch
+  // about a microsecond of host time (used under the plan's mutex)
+  struct BandMap {
+    const void *ptr = nullptr;
+    int ncol = 0, lgcw = 0;
+    CUtensorMap map;
+  };
+  mutable BandMap band_map[2];
 
   // host copies
   std::vector<double> h_mu, h_wgt;
@@ -193,12 +202,14 @@ int launch_fft_inv(const sht_plan *p, const double2 *F, int ncolF, int colF0, in
                    double *g0, double *g1, int nsplit, int rs, cudaStream_t s,
                    double *const *ocol = nullptr);
 
-// --- Legendre contraction, FP64 (sht_legendre.cu)
-int pick_fp64_kernel(const sht_plan *p);  // 1 per-band, 2 paired, 3 latitude-chunked
+// --- Legendre contraction, FP64: one band and parity per block, any grid
+// (sht_legendre_band.cu)
+int plan_band_items(sht_plan *p, std::vector<long long> &boff, std::vector<BandItem> &items);
+int build_band_table(sht_plan *p);
+int band_error_status(sht_plan *p);  // reads and clears the plan's error word (after a synchronisation)
 int launch_leg_fwd_fp64(const sht_plan *p, const double2 *F, int ncol, double2 *S, cudaStream_t s);
 int launch_leg_inv_fp64(const sht_plan *p, const double2 *S, int ncol, double2 *F, cudaStream_t s);
 
-// --- persistent paired-band FP64 contraction (sht_legendre_v2.cu)
 bool split_supported(const sht_plan *p);
 // Whether a contraction runs in split precision: always under SHT_PREC_SPLIT;
 // under SHT_PREC_AUTO when it is at least 128 terms long (jm/2 latitudes in
@@ -237,21 +248,6 @@ inline int grid_sms(const sht_plan *p)
   const int n = p->num_sms > 0 ? p->num_sms : 1;
   return (p->sm_cap > 0 && p->sm_cap < n) ? p->sm_cap : n;
 }
-bool leg_pair_supported(const sht_plan *p);
-int launch_leg_fwd_pair(const sht_plan *p, const double2 *F, int ncol, double2 *S, cudaStream_t s);
-int launch_leg_inv_pair(const sht_plan *p, const double2 *S, int ncol, double2 *F, cudaStream_t s);
-
-// --- one band and parity per block, any grid (sht_legendre_band.cu)
-int plan_band_items(sht_plan *p, std::vector<long long> &boff, std::vector<BandItem> &items);
-int build_band_table(sht_plan *p);
-int band_error_status(sht_plan *p);  // reads and clears the plan's error word (after a synchronisation)
-int launch_leg_fwd_band(const sht_plan *p, const double2 *F, int ncol, double2 *S, cudaStream_t s);
-int launch_leg_inv_band(const sht_plan *p, const double2 *S, int ncol, double2 *F, cudaStream_t s);
-
-// --- persistent latitude-chunked FP64 contraction for large grids (sht_legendre_v3.cu)
-bool leg_chunk_supported(const sht_plan *p);
-int launch_leg_fwd_chunk(const sht_plan *p, const double2 *F, int ncol, double2 *S, cudaStream_t s);
-int launch_leg_inv_chunk(const sht_plan *p, const double2 *S, int ncol, double2 *F, cudaStream_t s);
 
 // --- Legendre contraction, split precision on tcgen05 (sht_legendre_tc.cu)
 int launch_leg_fwd_split(sht_plan *p, const double2 *F, int ncol, double2 *S, cudaStream_t s);

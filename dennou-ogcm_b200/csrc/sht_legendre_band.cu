@@ -51,7 +51,6 @@
 #include "sht_tc.cuh"
 
 #include <algorithm>
-#include <cuda.h>
 
 namespace sht {
 
@@ -531,8 +530,15 @@ EncodeTiled encode_tiled()
 // The data operand as a tensor.  Analysis: (re/im of a latitude, parity half,
 // column, order); synthesis: (re/im of a column, row parity, row pair).  The
 // strides are multiples of 16 bytes whatever the counts.
-int data_map(const sht_plan *p, const BandArgs &a, bool inv, CUtensorMap *map)
+int data_map(const sht_plan *p, const BandArgs &a, bool inv, const CUtensorMap **out)
 {
+  auto &slot = p->band_map[inv];
+  const void *ptr = inv ? a.Sc : a.F;
+  *out = &slot.map;
+  // a map is a function of the address and the counts alone
+  if (slot.ptr == ptr && slot.ncol == a.ncol && slot.lgcw == a.lgcw) return SHT_OK;
+  slot.ptr = nullptr;
+  CUtensorMap *map = &slot.map;
   const EncodeTiled enc = encode_tiled();
   if (!enc) { set_error("legendre: the driver has no cuTensorMapEncodeTiled"); return SHT_ERR_CUDA; }
   const cuuint64_t nc = (cuuint64_t)a.ncol, col = 16ull * p->J;
@@ -553,6 +559,9 @@ int data_map(const sht_plan *p, const BandArgs &a, bool inv, CUtensorMap *map)
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   }
   if (r != CUDA_SUCCESS) { set_error("legendre: tensor map encoding failed"); return SHT_ERR_CUDA; }
+  slot.ptr = ptr;
+  slot.ncol = a.ncol;
+  slot.lgcw = a.lgcw;
   return SHT_OK;
 }
 
@@ -576,7 +585,7 @@ int run_band(const sht_plan *p, BandArgs a, cudaStream_t s)
   const long long units = units_at(lg);
   if (units > 0x3fffffffLL) { set_error("legendre: too many field-levels for one call"); return SHT_ERR_TOO_LARGE; }
   a.nunits = (int)units;
-  CUtensorMap map;
+  const CUtensorMap *map = nullptr;
   const int rc = data_map(p, a, INV, &map);
   if (rc) return rc;
   auto kern = (1 << lg) == W ? k_leg_band<W, TM, NS, MINB, INV, false> : k_leg_band<W, TM, NS, MINB, INV, true>;
@@ -584,7 +593,7 @@ int run_band(const sht_plan *p, BandArgs a, cudaStream_t s)
   cudaError_t e = kernel_setup((const void *)kern, smem, 32 * W + 32, &occ);
   if (e != cudaSuccess) return cuda_fail(e, "legendre band smem attribute");
   const long long gr = (long long)(occ < 1 ? 1 : occ) * grid_sms(p);
-  kern<<<(unsigned)std::min(units, gr), 32 * W + 32, smem, s>>>(map, a);
+  kern<<<(unsigned)std::min(units, gr), 32 * W + 32, smem, s>>>(*map, a);
   count_launch();
   e = cudaGetLastError();
   return e == cudaSuccess ? SHT_OK : cuda_fail(e, "k_leg_band");
@@ -605,7 +614,7 @@ int launch_band(const sht_plan *p, BandArgs a, cudaStream_t s)
 
 }  // namespace
 
-int launch_leg_fwd_band(const sht_plan *p, const double2 *F, int ncol, double2 *S, cudaStream_t s)
+int launch_leg_fwd_fp64(const sht_plan *p, const double2 *F, int ncol, double2 *S, cudaStream_t s)
 {
   if (ncol <= 0) return SHT_OK;
   BandArgs a{};
@@ -614,7 +623,7 @@ int launch_leg_fwd_band(const sht_plan *p, const double2 *F, int ncol, double2 *
   return launch_band<false>(p, a, s);
 }
 
-int launch_leg_inv_band(const sht_plan *p, const double2 *S, int ncol, double2 *F, cudaStream_t s)
+int launch_leg_inv_fp64(const sht_plan *p, const double2 *S, int ncol, double2 *F, cudaStream_t s)
 {
   if (ncol <= 0) return SHT_OK;
   BandArgs a{};

@@ -183,21 +183,11 @@ int time_group(Group &g, int reps, float *ms)
 
 int tune_group(Group &g, bool allow_split)
 {
-  // kernel families and their tiles: analysis columns per item of the paired
-  // kernels, latitudes per chunk of the chunked kernels (a tile a kernel
-  // cannot take falls back to its automatic one and is timed again
-  // harmlessly), and the single-kernel transform of small grids
+  // the band kernels, the single-kernel transform of small grids, and split
+  // precision where allowed
   struct Cand { int precision, leg_kernel, leg_tile; };
   std::vector<Cand> cands;
-  if (leg_pair_supported(g.plan)) {
-    cands.push_back({SHT_PREC_FP64, 2, 8});
-    cands.push_back({SHT_PREC_FP64, 2, 16});
-  }
-  if (leg_chunk_supported(g.plan)) {
-    cands.push_back({SHT_PREC_FP64, 3, 16});
-    cands.push_back({SHT_PREC_FP64, 3, 32});
-  }
-  cands.push_back({SHT_PREC_FP64, 1, 0});
+  cands.push_back({SHT_PREC_FP64, 0, 0});
   if (small_supported(g.plan)) cands.push_back({SHT_PREC_FP64, 4, 0});  // one kernel per direction
   if (allow_split && split_supported(g.plan)) {
     cands.push_back({SHT_PREC_SPLIT, 0, 0});

@@ -78,8 +78,9 @@ SHT_API const char *sht_last_error(void);
 
 /* SpmlUtil_Init(iMax, jMax, kMax, nMax, tMax, RPlanet, np)
  * (SpmlUtil_mod.f90:192-241; wa_Initial at :218-223).
- * im: longitudes (even, 16..2048: powers of two take the four-step FFT, other
- * counts such as 96, 192, 320 or 640 a direct summation over longitudes),
+ * im: longitudes (even, 16..2048: powers of two take the four-step FFT,
+ * counts with factors 3 and 5 such as 96, 192, 320 or 640 a mixed-radix FFT,
+ * others a direct summation over longitudes),
  * or 1 for the axisymmetric model
  * (DOGCM_MODE_AXISYM, SpmlUtil_mod.f90:30-35,210-211: SPMODEL
  * wa_zonal_module, only the m = 0 modes, lm = nm + 1 with wa(n+1) = a_n^0);
@@ -124,9 +125,8 @@ SHT_API int sht_set_precision(sht_plan *plan, int mode);
 SHT_API int sht_get_precision(const sht_plan *plan, int *mode);
 
 /* Kernel choices (used by the autotuner and the tests; the defaults are
- * picked per grid).  SHT_OPT_LEGENDRE_KERNEL: 0 automatic, 1 per-band kernel
- * (any grid), 2 persistent paired-band kernel (T85 and smaller), 3 persistent
- * latitude-chunked paired-band kernel (jm/2 a multiple of 16, up to T341),
+ * picked per grid).  SHT_OPT_LEGENDRE_KERNEL: 0 automatic; 1, 2 and 3 are
+ * accepted and run the automatic kernels (they named earlier FP64 kernels);
  * 4 the whole plain analysis or synthesis (w_xy, xy_w and their batched
  * forms) in one kernel per call, Fourier coefficients kept on chip (power-of-
  * two im <= 128, jm/2 a multiple of 4, FP64; other operators keep the
@@ -140,13 +140,8 @@ SHT_API int sht_get_precision(const sht_plan *plan, int *mode);
  * is the number of graphs the plan holds. */
 #define SHT_OPT_HOST_GRAPHS 2
 #define SHT_OPT_HOST_GRAPH_COUNT 3
-/* SHT_OPT_LEGENDRE_TILE: the tile of the FP64 Legendre kernels (0 automatic).
- * Paired kernels: 8 or 16 complex columns per analysis item; chunked kernels:
- * 16 or 32 latitudes per streamed chunk.  A value the chosen kernel does not
- * take, or whose shared memory does not fit, falls back to the automatic
- * tile.  Results are identical for every tile (the same products in the same
- * order per output).  The batch tuner (sht_multi_build with autotune) times
- * the tiles with the kernel families. */
+/* SHT_OPT_LEGENDRE_TILE: 0, 8, 16 or 32, kept and returned; the FP64 Legendre
+ * kernels have no choice of tiles any more. */
 #define SHT_OPT_LEGENDRE_TILE 4
 SHT_API int sht_set_option(sht_plan *plan, int option, int value);
 SHT_API int sht_get_option(const sht_plan *plan, int option, int *value);
