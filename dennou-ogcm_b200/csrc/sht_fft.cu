@@ -22,20 +22,20 @@
 // access touches eight distinct bank groups.
 #include "sht_fft_tile.cuh"
 #include "sht_fft_mixed.cuh"
+#include "sht_fft_row.cuh"
 
 #include <type_traits>
 
 namespace sht {
 
+// These kernels take im = 16 and 32 and im = 2048, and the inverse of
+// im = 1024; the counts between run the kernels of sht_fft_row.cu.
+//
 // Forward transform, persistent over tiles (field-level, JT latitude rows).
 // Each thread loads its R1 elements of row r (stride R2) from global memory
 // straight into registers; the block's one shared buffer takes the transpose
-// and the output staging.  Staging the tile with cp.async as well, in a
-// second pair of buffers, cost blocks per SM and measured the same at T85 and
-// 7-18 % slower at T170/T341.  Up to 16-point first passes the plain
-// transform also holds the block's next tile in registers while it works on
-// this one (3 instead of 4 blocks per SM at T85; forward 53 -> 52 us at T85,
-// 0.314 -> 0.283 ms at T170, the same at T42).
+// and the output staging.  Up to 16-point first passes the plain transform
+// also holds the block's next tile in registers while it works on this one.
 // MUL: 0 plain, 1 product with the factor grid (FftArgs::mul), read the same way.
 template <int A, int B, int NT, int MUL>
 __global__ void __launch_bounds__(NT) k_fft_fwd(FftArgs a)
@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(NT) k_fft_fwd(FftArgs a)
 // Inverse transform, persistent over tiles; the Fourier runs of tile
 // t+gridDim.x stream into one buffer while tile t is transformed in place.
 template <int A, int B, int NT>
-__global__ void __launch_bounds__(NT, (A == 4 && B == 3) ? 4 : 1) k_fft_inv(FftArgs a, int bufe)
+__global__ void __launch_bounds__(NT) k_fft_inv(FftArgs a, int bufe)
 {
   using S = FftShape<A, B, NT>;
   constexpr int R1 = S::R1, R2 = S::R2, NC = S::NC, T = S::T, JT = S::JT, JTp = S::JTp;
@@ -150,10 +150,9 @@ __global__ void __launch_bounds__(NT, (A == 4 && B == 3) ? 4 : 1) k_fft_inv(FftA
   constexpr int JTh = JT / 2;  // mirrored row pairs per tile
   const int tid = threadIdx.x, r = tid / T, u = tid % T;
   const int ntile = (a.JH + JTh - 1) / JTh;
-  // Tile indices fit in 32 bits (the launcher checks).  Up to 16-point first
-  // passes the per-tile division is a 32-bit one (T85 / T170 inverse 1-4 %
-  // faster); at 32 points, where the kernel sits at the 255-register cap, the
-  // 64-bit form measured faster (T341 inverse 1.58 against 1.84 ms).
+  // Tile indices fit in 32 bits (the launcher checks).  At 32 points, where the
+  // kernel sits at the 255-register cap, the 64-bit form measured faster (T341
+  // inverse 1.58 against 1.84 ms).
   using Idx = typename std::conditional<(A <= 4), unsigned, long long>::type;
   const Idx ntot = (Idx)a.ncol * (Idx)ntile;
   const long long mstride = (long long)a.ncolF * a.J;
@@ -175,10 +174,8 @@ __global__ void __launch_bounds__(NT, (A == 4 && B == 3) ? 4 : 1) k_fft_inv(FftA
   // Up to 16-point first passes the next tile's runs stream into the second
   // buffer while this one is transformed.  At 32 points a buffer is 67 KB and
   // the kernel needs 254 registers: one buffer per block, so that two blocks
-  // share an SM and one block's loads overlap the other's transform.  At 128
-  // complex points (I = 256) one buffer and a 128-register cap give 4 blocks
-  // per SM instead of 3 (inverse 55.0 -> 53.9 us at T85, 480 field-levels).
-  constexpr bool kDB = A <= 4 && !(A == 4 && B == 3);
+  // share an SM and one block's loads overlap the other's transform.
+  constexpr bool kDB = A <= 4;
   Idx t = blockIdx.x;
   if (t < ntot) issue(t, sm);
   cp_async_commit();
@@ -438,14 +435,14 @@ int run_dft(bool inverse, const sht_plan *p, const FftArgs &a, cudaStream_t s)
 
 // Persistent grids: as many blocks as fit on the device at once, never more
 // than there are tiles.
-template <int A, int B>
+template <int A, int B, bool FWD = true>
 int run_fft(bool inverse, const sht_plan *p, const FftArgs &a, cudaStream_t s)
 {
   using S = FftShape<A, B, kFftThreads>;
   // inverse up to 16-point first passes: two buffers (staged Fourier runs of
   // the next tile beside the current one); otherwise one buffer
   const int bufe = S::buf_elems(p->N);
-  const size_t smem = sizeof(double2) * (2 * (size_t)S::NC + (inverse && A <= 4 && !(A == 4 && B == 3) ? 2 : 1) * (size_t)bufe);
+  const size_t smem = sizeof(double2) * (2 * (size_t)S::NC + (inverse && A <= 4 ? 2 : 1) * (size_t)bufe);
   const long long ntiles = (long long)a.ncol * ((p->JH + S::JT / 2 - 1) / (S::JT / 2));
   if (ntiles <= 0) return SHT_OK;
   if (ntiles > 0x7fffffffLL) { set_error("fft: too many field-levels for one call"); return SHT_ERR_TOO_LARGE; }
@@ -457,9 +454,12 @@ int run_fft(bool inverse, const sht_plan *p, const FftArgs &a, cudaStream_t s)
     const long long g = (long long)(occ < 1 ? 1 : occ) * grid_sms(p);
     kern<<<(int)(ntiles < g ? ntiles : g), kFftThreads, smem, s>>>(a, extra...);
   };
-  if (inverse) go(k_fft_inv<A, B, kFftThreads>, bufe);
-  else if (a.mul) go(k_fft_fwd<A, B, kFftThreads, 1>);
-  else go(k_fft_fwd<A, B, kFftThreads, 0>);
+  if (inverse) {
+    go(k_fft_inv<A, B, kFftThreads>, bufe);
+  } else if constexpr (FWD) {
+    if (a.mul) go(k_fft_fwd<A, B, kFftThreads, 1>);
+    else go(k_fft_fwd<A, B, kFftThreads, 0>);
+  }
   if (e != cudaSuccess) return cuda_fail(e, "fft smem attribute");
   count_launch();
   e = cudaGetLastError();
@@ -481,14 +481,11 @@ int dispatch(bool inverse, const sht_plan *p, const FftArgs &args, cudaStream_t 
   }
   // factors 3 and 5: the mixed-radix FFT; other prime factors: the direct sum
   if (p->direct_dft) return fft_mixed_supported(p->I, p->N) ? run_fft_mixed(inverse, p, args, s) : run_dft(inverse, p, args, s);
+  if (fft_row_supported(p->NC, inverse)) return run_fft_row(inverse, p, args, s);
   switch (p->NC) {
   case 8: return run_fft<2, 1>(inverse, p, args, s);
   case 16: return run_fft<2, 2>(inverse, p, args, s);
-  case 32: return run_fft<3, 2>(inverse, p, args, s);
-  case 64: return run_fft<3, 3>(inverse, p, args, s);
-  case 128: return run_fft<4, 3>(inverse, p, args, s);
-  case 256: return run_fft<4, 4>(inverse, p, args, s);
-  case 512: return run_fft<5, 4>(inverse, p, args, s);
+  case 512: return run_fft<5, 4, false>(inverse, p, args, s);
   case 1024: return run_fft<5, 5>(inverse, p, args, s);
   default: set_error("fft: unsupported longitude count"); return SHT_ERR_UNSUPPORTED_SIZE;
   }
