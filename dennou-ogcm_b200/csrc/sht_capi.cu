@@ -1195,18 +1195,20 @@ int sht_synthesis_dev(sht_plan *p, const double *wa, int ldw, int nb, double *xy
   return strided_call(p, false, nullptr, xya, ldi, ldj, nb, wa, nullptr, ldw, mode, false);
 }
 
-static int diffuse_impl(sht_plan *p, double *w, int nb, const double *coef, double dt, const double *filter, bool host)
+// w: the spectra; out: the device result (w itself in place; unused by host calls, which are in place)
+static int diffuse_impl(sht_plan *p, const double *w, int nb, const double *coef, double dt, const double *filter,
+                        double *out, bool host)
 {
   int rc = check_plan(p);
   if (rc) return rc;
-  if (nb < 0 || (nb > 0 && (!w || !coef))) { set_error("diffuse: bad argument"); return SHT_ERR_INVALID_ARG; }
+  if (nb < 0 || (nb > 0 && (!w || !coef || !out))) { set_error("diffuse: bad argument"); return SHT_ERR_INVALID_ARG; }
   if (nb == 0) return SHT_OK;
   std::lock_guard<std::mutex> lk(p->mtx);
   DeviceGuard g(p->device);
   if (!g.ok) { set_error("cudaSetDevice failed"); return SHT_ERR_CUDA; }
   cudaStream_t s = p->stream;
   cudaError_t e;
-  if (!host) return launch_diffuse(p, w, nb, coef, dt, filter, s);
+  if (!host) return launch_diffuse(p, w, nb, coef, dt, filter, out, s);
   const size_t nw = (size_t)nb * p->L;
   if ((rc = ensure_io(p, sizeof(double) * (nw + 2 * p->L) + 1024))) return rc;
   double *dw = static_cast<double *>(p->d_io), *dc = dw + nw, *df = dc + p->L;
@@ -1214,16 +1216,19 @@ static int diffuse_impl(sht_plan *p, double *w, int nb, const double *coef, doub
       (e = cudaMemcpyAsync(dc, coef, sizeof(double) * p->L, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
       (filter && (e = cudaMemcpyAsync(df, filter, sizeof(double) * p->L, cudaMemcpyHostToDevice, s)) != cudaSuccess))
     return cuda_fail(e, "H2D");
-  if ((rc = launch_diffuse(p, dw, nb, dc, dt, filter ? df : nullptr, s))) return rc;
-  if ((e = cudaMemcpyAsync(w, dw, sizeof(double) * nw, cudaMemcpyDeviceToHost, s)) != cudaSuccess) return cuda_fail(e, "D2H");
+  if ((rc = launch_diffuse(p, dw, nb, dc, dt, filter ? df : nullptr, dw, s))) return rc;
+  if ((e = cudaMemcpyAsync(out, dw, sizeof(double) * nw, cudaMemcpyDeviceToHost, s)) != cudaSuccess) return cuda_fail(e, "D2H");
   if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_fail(e, "diffuse");
   return SHT_OK;
 }
 
 int sht_wa_diffuse(sht_plan *p, double *w, int nb, const double *coef, double dt, const double *filter)
-{ return diffuse_impl(p, w, nb, coef, dt, filter, true); }
+{ return diffuse_impl(p, w, nb, coef, dt, filter, w, true); }
 int sht_wa_diffuse_dev(sht_plan *p, double *w, int nb, const double *coef, double dt, const double *filter)
-{ return diffuse_impl(p, w, nb, coef, dt, filter, false); }
+{ return diffuse_impl(p, w, nb, coef, dt, filter, w, false); }
+int sht_wa_diffuse_to_dev(sht_plan *p, const double *w, int nb, const double *coef, double dt, const double *filter,
+                          double *out)
+{ return diffuse_impl(p, w, nb, coef, dt, filter, out, false); }
 
 int sht_roundtrip_diffuse_dev(sht_plan *p, double *xya, int nb, const double *coef, double dt, const double *filter)
 {
@@ -1238,7 +1243,7 @@ int sht_roundtrip_diffuse_dev(sht_plan *p, double *xya, int nb, const double *co
   Workspace ws{};
   if ((rc = ensure_ws(p, nb, nb, &ws))) return rc;
   if ((rc = run_analysis(p, PACK_PLAIN, RS_FWD_PLAIN, xya, nullptr, nb, ws.W, nullptr))) return rc;
-  if (coef && (rc = launch_diffuse(p, ws.W, nb, coef, dt, filter, p->stream))) return rc;
+  if (coef && (rc = launch_diffuse(p, ws.W, nb, coef, dt, filter, ws.W, p->stream))) return rc;
   return run_synthesis(p, UNPACK_PLAIN, RS_INV_PLAIN, ws.W, nullptr, nb, xya, nullptr);
 }
 

@@ -112,6 +112,7 @@ def load_library(path: str | None = None):
                                                        ctypes.c_int, ctypes.c_int]
         getattr(lib, "sht_synthesis" + suf).argtypes = [_VP, _VP, ctypes.c_int, ctypes.c_int, _VP, ctypes.c_int,
                                                         ctypes.c_int, ctypes.c_int]
+    lib.sht_wa_diffuse_to_dev.argtypes = [_VP, _VP, ctypes.c_int, _VP, ctypes.c_double, _VP, _VP]
     lib.sht_roundtrip_diffuse_dev.argtypes = [_VP, _VP, ctypes.c_int, _VP, ctypes.c_double, _VP]
     lib.sht_plan_l_nm.argtypes = [_VP, ctypes.c_int, ctypes.c_int]
     lib.sht_plan_nm_l.argtypes = [_VP, ctypes.c_int, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int)]
@@ -430,10 +431,12 @@ class SpmlUtil:
         lib = load_library()
         nb, batched = self._spec_shape(wa)
         if _is_torch_cuda(wa):
-            out = wa.contiguous().clone()
+            import torch
+            x = wa.contiguous()
+            out = torch.empty_like(x)
             self._set_torch_stream(out)
-            st = lib.sht_wa_diffuse_dev(self._h, _VP(out.data_ptr()), nb, _VP(coef.data_ptr()), float(dt),
-                                        _VP(filt.data_ptr()) if filt is not None else None)
+            st = lib.sht_wa_diffuse_to_dev(self._h, _VP(x.data_ptr()), nb, _VP(coef.data_ptr()), float(dt),
+                                           _VP(filt.data_ptr()) if filt is not None else None, _VP(out.data_ptr()))
         else:
             out = np.array(wa, dtype=np.float64, copy=True, order="C")
             c = np.ascontiguousarray(coef, dtype=np.float64)

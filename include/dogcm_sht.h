@@ -302,6 +302,9 @@ SHT_API int sht_wa_lapla_wa_dev(sht_plan *plan, const double *wa, int nb, double
 SHT_API int sht_wa_laplainv_wa_dev(sht_plan *plan, const double *wa, int nb, double *out);
 SHT_API int sht_wa_diffuse_dev(sht_plan *plan, double *wa, int nb, const double *coef, double dt,
                        const double *filter);
+/* the same into another array (out may be wa) */
+SHT_API int sht_wa_diffuse_to_dev(sht_plan *plan, const double *wa, int nb, const double *coef, double dt,
+                          const double *filter, double *out);
 SHT_API int sht_avrlonlat_xya_dev(sht_plan *plan, const double *xya, int nb, double *out);
 SHT_API int sht_intlonlat_xya_dev(sht_plan *plan, const double *xya, int nb, double *out);
 SHT_API int sht_ya_avrlon_xya_dev(sht_plan *plan, const double *xya, int nb, double *out);
