@@ -94,10 +94,15 @@ __global__ void __launch_bounds__(256) k_pack(SpecArgs a)
   // every load of the thread is issued before any is used: out-of-range
   // entries read element 0 and are replaced by zero
   double2 c[NI][3][2];
+  double ev[NI][2];  // eps_n^m and eps_{n+1}^m, loaded with the coefficients
 #pragma unroll
   for (int i = 0; i < NI; ++i) {
     const int m = m0 + warp + 8 * i;
     const bool ok = m <= n && m < a.M && b < a.nb;
+    if (OP != PACK_PLAIN && OP != PACK_DIVLAMBDA) {
+      ev[i][0] = ok ? eps_at(a, m, n) : 0.0;
+      ev[i][1] = ok ? eps_at(a, m, n + 1) : 0.0;
+    }
     const long long base = ok ? (long long)spec_row(a.N, m, n) * a.ncolS + b : 0;
 #pragma unroll
     for (int dn = -1; dn <= 1; ++dn)
@@ -116,7 +121,7 @@ __global__ void __launch_bounds__(256) k_pack(SpecArgs a)
     double2 v0 = make_double2(0.0, 0.0), v1 = make_double2(0.0, 0.0);
     if (m <= n && m < a.M && b < a.nb) {
       auto D = [&](int set) -> double2 {  // -( (n+1) eps_n c_{n-1} - n eps_{n+1} c_{n+1} )
-        const double e0 = (n + 1) * eps_at(a, m, n), e1 = n * eps_at(a, m, n + 1);
+        const double e0 = (n + 1) * ev[i][0], e1 = n * ev[i][1];
         const double2 cm = c[i][0][set], cp = c[i][2][set];
         return make_double2(e1 * cp.x - e0 * cm.x, e1 * cp.y - e0 * cm.y);
       };
@@ -171,35 +176,37 @@ __host__ __device__ constexpr bool unpack_needs(int in, int dn)
                                                       : true;  // VORDIV2UV
 }
 template <int OP>
-__host__ __device__ constexpr int unpack_slot(int run)  // compact shared-memory slot of a needed run
-{
-  int s = 0;
-  for (int r = 0; r < run; ++r) s += unpack_needs<OP>(r / 6, (r % 6) / 2 - 1) ? 1 : 0;
-  return s;
-}
-template <int OP>
-__host__ __device__ constexpr int unpack_nslots() { return unpack_slot<OP>(12); }
+__host__ __device__ constexpr int unpack_outputs() { return OP == UNPACK_VORDIV2UV || OP == UNPACK_HGRAD ? 2 : 1; }
 
+// A warp takes field-levels b0 + 8 i' + w with its lanes along the orders
+// (256-byte runs of the SPML rows), applies the operator there, and stages
+// only the results, transposed, for stores with the lanes along the
+// field-levels.  Staging the entries instead (up to twelve runs, 101 KB for
+// U, V from vorticity and divergence) and dividing by n(n+1) in every
+// thread's inner loop took 63 us for that operator at T85 with 480 levels, 41
+// now (116 MB).
 template <int OP>
 __global__ void __launch_bounds__(256) k_unpack(SpecArgs a)
 {
   constexpr int NIN = (OP == UNPACK_ALPHA || OP == UNPACK_VORDIV2UV) ? 2 : 1;
-  extern __shared__ double ws_dyn[];  // [slot][m][b]
-  auto ws = reinterpret_cast<double(*)[kMC][kBC + 1]>(ws_dyn);
+  constexpr int NOUT = unpack_outputs<OP>();
+  constexpr bool kEps = OP != UNPACK_PLAIN && OP != UNPACK_GRADLAMBDA;
+  __shared__ double ws[2 * NOUT][kMC][kBC + 1];  // [output, re/im][m][b]
   const int2 t = a.tiles[blockIdx.x];
   const int n = t.x, m0 = t.y;
   const int b0 = blockIdx.y * kBC;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // Stage the SPML entries the operator reads (degrees n-1..n+1 as needed,
-  // orders m0..m0+31, both parts).  Warp w takes field-levels b0 + 8i' + w of
-  // every run, so the run of each unrolled load is a compile-time constant;
-  // all loads of a warp are issued before any of them is stored.
   constexpr int NQ = kBC / 8;
-  constexpr int PER = NIN * 6 * NQ;
-  double val[PER];
   const int m = m0 + lane;
-  // the row of each of this warp's field-levels, and the SPML offset of each
-  // run (-1 where the entry does not exist), formed once for all loads
+  // the SPML offset of each run (dn = -1..1, cos/sin part; -1 where the entry
+  // does not exist) and the recurrence's coefficients, formed once
+  int off[6];
+#pragma unroll
+  for (int r = 0; r < 6; ++r) {
+    const int nn = n + r / 2 - 1, sn = r & 1;
+    const bool ok = nn >= 0 && nn <= a.N && m <= nn && m < a.M && !(sn && m == 0);
+    off[r] = ok ? (int)spml_l(a, nn, m, sn) : -1;
+  }
   const double *wr[NIN][NQ];
 #pragma unroll
   for (int in = 0; in < NIN; ++in)
@@ -209,55 +216,44 @@ __global__ void __launch_bounds__(256) k_unpack(SpecArgs a)
       wr[in][q] = bb >= a.nb ? nullptr
                 : (in == 0 && a.icol) ? a.icol[bb] : ((in == 0) ? a.w0 : a.w1) + (long long)bb * a.L;
     }
-  int off[6];
+  double x[NQ][NIN][3][2];
 #pragma unroll
-  for (int r = 0; r < 6; ++r) {
-    const int nn = n + r / 2 - 1, sn = r & 1;
-    const bool ok = nn >= 0 && nn <= a.N && m <= nn && m < a.M && !(sn && m == 0);
-    off[r] = ok ? (int)spml_l(a, nn, m, sn) : -1;
+  for (int in = 0; in < NIN; ++in)
+#pragma unroll
+    for (int r = 0; r < 6; ++r)
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+        x[q][in][r / 2][r & 1] = 0.0;
+        if (!unpack_needs<OP>(in, r / 2 - 1)) continue;
+        const double *w = wr[in][q];
+        const int o = off[r];
+        if (w && o >= 0) x[q][in][r / 2][r & 1] = __ldg(w + o);
+      }
+  const bool mok = m <= n && m <= a.N && m < a.M;
+  double ep = 0.0, em = 0.0;  // R(x)_n = (n+2) eps_{n+1} x_{n+1} - (n-1) eps_n x_{n-1}
+  if (kEps && mok) {
+    ep = (n + 2) * eps_at(a, m, n + 1);
+    em = (n - 1) * eps_at(a, m, n);
   }
+  // -a^2/(k(k+1)) for the degrees n - 1, n, n + 1
+  double lap[3] = {0.0, 0.0, 0.0};
+  if constexpr (OP == UNPACK_VORDIV2UV) {
+    const double a2 = a.radius * a.radius;
 #pragma unroll
-  for (int i = 0; i < PER; ++i) {
-    const int run = i / NQ;
-    val[i] = 0.0;
-    if (!unpack_needs<OP>(run / 6, (run % 6) / 2 - 1)) continue;
-    const double *w = wr[run / 6][i % NQ];
-    const int o = off[run % 6];
-    if (w && o >= 0) val[i] = __ldg(w + o);
+    for (int d = 0; d < 3; ++d) {
+      const double k = n + d - 1.0;
+      lap[d] = k >= 1.0 ? -a2 / (k * (k + 1.0)) : 0.0;
+    }
   }
+  const double s = (m == 0) ? 1.0 : kRSqrt2;
 #pragma unroll
-  for (int i = 0; i < PER; ++i) {
-    const int run = i / (kBC / 8);
-    if (unpack_needs<OP>(run / 6, (run % 6) / 2 - 1))
-      ws[unpack_slot<OP>(run)][lane][8 * (i % (kBC / 8)) + warp] = val[i];
-  }
-  __syncthreads();
-  const int b = b0 + lane;
-  if (b >= a.nb) return;
-  int rows[kMC / 8];  // internal rows of this warp's orders
-#pragma unroll
-  for (int i = 0; i < kMC / 8; ++i) {
-    const int m = m0 + warp + 8 * i;
-    rows[i] = (m <= n && m <= a.N && m < a.M) ? spec_row(a.N, m, n) : -1;
-  }
-#pragma unroll
-  for (int i = 0; i < kMC / 8; ++i) {
-    const int mi = warp + 8 * i, m = m0 + mi;
-    if (rows[i] < 0) continue;
-    const double s = (m == 0) ? 1.0 : kRSqrt2;
-    auto coef = [&](int in, int dn) -> double2 {
-      const int run = in * 6 + (dn + 1) * 2;
-      return make_double2(ws[unpack_slot<OP>(run)][mi][lane] * s, ws[unpack_slot<OP>(run + 1)][mi][lane] * s);
-    };
-    auto R = [&](int in, double mult0) -> double2 {  // (n+2) eps_{n+1} x_{n+1} - (n-1) eps_n x_{n-1}, x scaled per degree
-      const double ep = (n + 2) * eps_at(a, m, n + 1), em = (n - 1) * eps_at(a, m, n);
+  for (int q = 0; q < NQ; ++q) {
+    auto coef = [&](int in, int dn) { return make_double2(x[q][in][dn + 1][0] * s, x[q][in][dn + 1][1] * s); };
+    auto R = [&](int in, bool inv_lap) {
       double2 xp = coef(in, 1), xm = coef(in, -1);
-      if (mult0 != 0.0) {  // inverse Laplacian scaling -a^2/(k(k+1)) per degree
-        const double kp = n + 1.0, km = n - 1.0;
-        const double sp = -mult0 / (kp * (kp + 1.0));
-        const double sm_ = (km >= 1.0) ? -mult0 / (km * (km + 1.0)) : 0.0;
-        xp = cscale(xp, sp);
-        xm = cscale(xm, sm_);
+      if (inv_lap) {
+        xp = cscale(xp, lap[2]);
+        xm = cscale(xm, lap[0]);
       }
       return make_double2(ep * xp.x - em * xm.x, ep * xp.y - em * xm.y);
     };
@@ -267,22 +263,40 @@ __global__ void __launch_bounds__(256) k_unpack(SpecArgs a)
     } else if (OP == UNPACK_GRADLAMBDA) {
       v0 = times_im(coef(0, 0), m);
     } else if (OP == UNPACK_GRADMU) {
-      v0 = R(0, 0.0);
+      v0 = R(0, false);
     } else if (OP == UNPACK_HGRAD) {
       v0 = times_im(coef(0, 0), m);
-      v1 = R(0, 0.0);
+      v1 = R(0, false);
     } else if (OP == UNPACK_ALPHA) {
-      v0 = cadd(times_im(coef(0, 0), m), R(1, 0.0));
+      v0 = cadd(times_im(coef(0, 0), m), R(NIN - 1, false));
     } else {  // UNPACK_VORDIV2UV: input 0 = vor, 1 = div
-      const double a2 = a.radius * a.radius;
-      const double sn = (n >= 1) ? -a2 / ((double)n * (n + 1.0)) : 0.0;
-      const double2 psi = cscale(coef(0, 0), sn), chi = cscale(coef(1, 0), sn);
-      v0 = csub(times_im(chi, m), R(0, a2));
-      v1 = cadd(times_im(psi, m), R(1, a2));
+      const double2 psi = cscale(coef(0, 0), lap[1]), chi = cscale(coef(NIN - 1, 0), lap[1]);
+      v0 = csub(times_im(chi, m), R(0, true));
+      v1 = cadd(times_im(psi, m), R(NIN - 1, true));
     }
-    const long long row = rows[i];
-    a.So[row * a.ncolS + b] = v0;
-    if (OP == UNPACK_VORDIV2UV || OP == UNPACK_HGRAD) a.So[row * a.ncolS + a.nb + b] = v1;
+    ws[0][lane][8 * q + warp] = v0.x;
+    ws[1][lane][8 * q + warp] = v0.y;
+    if constexpr (NOUT == 2) {
+      ws[2][lane][8 * q + warp] = v1.x;
+      ws[3][lane][8 * q + warp] = v1.y;
+    }
+  }
+  __syncthreads();
+  const int b = b0 + lane;
+  if (b >= a.nb) return;
+  int rows[kMC / 8];  // internal rows of this warp's orders
+#pragma unroll
+  for (int i = 0; i < kMC / 8; ++i) {
+    const int mw = m0 + warp + 8 * i;
+    rows[i] = (mw <= n && mw <= a.N && mw < a.M) ? spec_row(a.N, mw, n) : -1;
+  }
+#pragma unroll
+  for (int i = 0; i < kMC / 8; ++i) {
+    const int mi = warp + 8 * i;
+    if (rows[i] < 0) continue;
+    double2 *So = a.So + (long long)rows[i] * a.ncolS + b;
+    So[0] = make_double2(ws[0][mi][lane], ws[1][mi][lane]);
+    if constexpr (NOUT == 2) So[a.nb] = make_double2(ws[2][mi][lane], ws[3][mi][lane]);
   }
 }
 
@@ -394,25 +408,17 @@ int launch_unpack(const sht_plan *p, int op, const double *w0, const double *w1,
   a.eps = p->d_eps; a.tiles = p->d_spec_tiles;
   a.M = p->M; a.zonal = p->zonal ? 1 : 0;
   dim3 grid(p->n_spec_tiles, (nb + kBC - 1) / kBC);
-  const size_t one = sizeof(double) * kMC * (kBC + 1);  // one staged run
-  cudaError_t e = cudaSuccess;
-  auto run = [&](auto kern, int nslots) {
-    const size_t smem = one * nslots;
-    e = kernel_setup((const void *)kern, smem, 256);
-    if (e == cudaSuccess) kern<<<grid, 256, smem, s>>>(a);
-  };
   switch (op) {
-  case UNPACK_PLAIN: run(k_unpack<UNPACK_PLAIN>, unpack_nslots<UNPACK_PLAIN>()); break;
-  case UNPACK_GRADLAMBDA: run(k_unpack<UNPACK_GRADLAMBDA>, unpack_nslots<UNPACK_GRADLAMBDA>()); break;
-  case UNPACK_GRADMU: run(k_unpack<UNPACK_GRADMU>, unpack_nslots<UNPACK_GRADMU>()); break;
-  case UNPACK_ALPHA: run(k_unpack<UNPACK_ALPHA>, unpack_nslots<UNPACK_ALPHA>()); break;
-  case UNPACK_VORDIV2UV: run(k_unpack<UNPACK_VORDIV2UV>, unpack_nslots<UNPACK_VORDIV2UV>()); break;
-  case UNPACK_HGRAD: run(k_unpack<UNPACK_HGRAD>, unpack_nslots<UNPACK_HGRAD>()); break;
+  case UNPACK_PLAIN: k_unpack<UNPACK_PLAIN><<<grid, 256, 0, s>>>(a); break;
+  case UNPACK_GRADLAMBDA: k_unpack<UNPACK_GRADLAMBDA><<<grid, 256, 0, s>>>(a); break;
+  case UNPACK_GRADMU: k_unpack<UNPACK_GRADMU><<<grid, 256, 0, s>>>(a); break;
+  case UNPACK_ALPHA: k_unpack<UNPACK_ALPHA><<<grid, 256, 0, s>>>(a); break;
+  case UNPACK_VORDIV2UV: k_unpack<UNPACK_VORDIV2UV><<<grid, 256, 0, s>>>(a); break;
+  case UNPACK_HGRAD: k_unpack<UNPACK_HGRAD><<<grid, 256, 0, s>>>(a); break;
   default: set_error("unpack: unknown operator"); return SHT_ERR_INVALID_ARG;
   }
-  if (e != cudaSuccess) return cuda_fail(e, "k_unpack smem attribute");
   count_launch();
-  e = cudaGetLastError();
+  cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? SHT_OK : cuda_fail(e, "k_unpack");
 }
 
