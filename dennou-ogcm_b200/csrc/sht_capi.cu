@@ -215,6 +215,12 @@ int run_analysis(sht_plan *p, int pack_op, int rs, const double *g0, const doubl
   mark(p, 0, s);
   if ((rc = launch_fft_fwd(p, g0, g1, nb, ncol, ws.F, ncol, 0, rs, s, nullptr, mul, nb, add0, add1))) return rc;
   mark(p, 1, s);
+  if (!use_split(p, true) && use_narrow(p, nb, nin)) {
+    // contraction and conversion in one kernel (timed as the contraction)
+    if ((rc = launch_narrow_fwd(p, pack_op, ws.F, ncol, nb, w0, w1, s))) return rc;
+    mark(p, 2, s); mark(p, 3, s);
+    return SHT_OK;
+  }
   if ((rc = leg_fwd(p, ws.F, ncol, ws.S, s))) return rc;
   mark(p, 2, s);
   if ((rc = launch_pack(p, pack_op, ws.S, ncol, nb, w0, w1, s))) return rc;
@@ -239,9 +245,14 @@ int run_synthesis(sht_plan *p, int unpack_op, int rs, const double *w0, const do
   Workspace ws{};
   if ((rc = ensure_ws(p, ncol, 0, &ws))) return rc;
   mark(p, 0, s);
-  if ((rc = launch_unpack(p, unpack_op, w0, w1, nb, ws.S, ncol, s))) return rc;
-  mark(p, 1, s);
-  if ((rc = leg_inv(p, ws.S, ncol, ws.F, s))) return rc;
+  if (!use_split(p, false) && use_narrow(p, nb, nout)) {
+    mark(p, 1, s);  // conversion and contraction in one kernel (timed as the contraction)
+    if ((rc = launch_narrow_inv(p, unpack_op, w0, w1, nb, ws.F, ncol, s))) return rc;
+  } else {
+    if ((rc = launch_unpack(p, unpack_op, w0, w1, nb, ws.S, ncol, s))) return rc;
+    mark(p, 1, s);
+    if ((rc = leg_inv(p, ws.S, ncol, ws.F, s))) return rc;
+  }
   mark(p, 2, s);
   if ((rc = launch_fft_inv(p, ws.F, ncol, 0, ncol, g0, g1, nb, rs, s))) return rc;
   mark(p, 3, s);

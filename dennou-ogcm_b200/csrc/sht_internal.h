@@ -267,6 +267,14 @@ int run_analysis_cols(sht_plan *p, const double *const *gcol, int ncol, double *
 int run_synthesis_cols(sht_plan *p, const double *const *wcol, int ncol, double *const *gcol, double2 *F,
                        double2 *S, cudaStream_t s);
 
+// --- contraction and layout conversion in one kernel, narrow batches
+// (sht_narrow.cu): sets is the operator's inputs (analysis) or outputs
+// (synthesis), ncol = sets nb the columns of F
+bool use_narrow(const sht_plan *p, int nb, int sets);
+int launch_narrow_fwd(const sht_plan *p, int op, const double2 *F, int ncol, int nb, double *w0, double *w1, cudaStream_t s);
+int launch_narrow_inv(const sht_plan *p, int op, const double *w0, const double *w1, int nb, double2 *F, int ncol,
+                      cudaStream_t s);
+
 // --- spectral-side kernels (sht_spectral.cu)
 // internal S (ncolS columns; set A at col 0, set B at col nb) -> SPML wa outputs
 // (field-level b at w0 + b L, or at wcol[b] when a column table is given;

@@ -23,63 +23,16 @@
 //
 // Both conversions tile by (total degree n, a chunk of 32 orders m, 32
 // field-levels) so that global reads and writes are 256-512 byte runs.
-#include "sht_internal.h"
+#include "sht_spectral.cuh"
 
 namespace sht {
 
 namespace {
+
+using namespace spec;
+
 constexpr int kMC = 32;  // orders per tile
 constexpr int kBC = 32;  // field-levels per tile
-constexpr double kSqrt2 = 1.41421356237309504880;
-constexpr double kRSqrt2 = 0.70710678118654752440;
-
-struct SpecArgs {
-  const double2 *S;   // pack input
-  double2 *So;        // unpack output
-  int ncolS;
-  const double *w0, *w1;  // unpack inputs
-  double *o0, *o1;        // pack outputs
-  int nb, N, L;
-  double radius;
-  const double *eps;      // [m][n], n = 0..N+2
-  const int2 *tiles;      // (n, m0) per tile
-  double *const *ocol;        // optional per-field-level pack destinations
-  const double *const *icol;  // optional per-field-level unpack sources
-  int M;                      // orders present: N + 1, or 1 for a zonal plan
-  int zonal;                  // SPML index l = n (wa_zonal_module) instead of n(n+1) +- m
-};
-
-// 0-based SPML index of (n, m), cos (sn = 0) or sin (sn = 1) part
-__device__ __forceinline__ long long spml_l(const SpecArgs &a, int n, int m, int sn)
-{
-  return a.zonal ? (long long)n : (long long)n * (n + 1) + (sn ? -m : m);
-}
-
-__device__ __forceinline__ double eps_at(const SpecArgs &a, int m, int n)
-{
-  return (n < 0 || n > a.N + 2) ? 0.0 : __ldg(a.eps + (long long)m * (a.N + 3) + n);
-}
-
-// Internal row of (m, n): rowoff(m) + n - m, with rowoff(m) = sum over m' < m
-// of the N + 2 - m' rows of band m' (the plan's row table in closed form, so
-// that no dependent load precedes the coefficient loads)
-__device__ __forceinline__ int spec_row(int N, int m, int n) { return m * (N + 2) - m * (m - 1) / 2 + (n - m); }
-__device__ __forceinline__ double2 cadd(double2 x, double2 y) { return make_double2(x.x + y.x, x.y + y.y); }
-__device__ __forceinline__ double2 csub(double2 x, double2 y) { return make_double2(x.x - y.x, x.y - y.y); }
-__device__ __forceinline__ double2 cscale(double2 x, double s) { return make_double2(x.x * s, x.y * s); }
-__device__ __forceinline__ double2 times_im(double2 x, int m) { return make_double2(-m * x.y, m * x.x); }
-
-// Which internal rows a pack operator reads: degree offset dn in -1..1 of
-// column set `set` (0: the first input's columns, 1: the second's).
-template <int OP>
-__host__ __device__ constexpr bool pack_needs(int dn, int set)
-{
-  return OP == PACK_PLAIN || OP == PACK_DIVLAMBDA ? (dn == 0 && set == 0)
-       : OP == PACK_DIVMU                         ? (dn != 0 && set == 0)
-       : OP == PACK_ALPHA                         ? (set == 0 ? dn == 0 : dn != 0)
-                                                  : true;  // VORDIV
-}
-
 template <int OP>
 __global__ void __launch_bounds__(256) k_pack(SpecArgs a)
 {
@@ -119,25 +72,7 @@ __global__ void __launch_bounds__(256) k_pack(SpecArgs a)
   for (int i = 0; i < NI; ++i) {
     const int mi = warp + 8 * i, m = m0 + mi;
     double2 v0 = make_double2(0.0, 0.0), v1 = make_double2(0.0, 0.0);
-    if (m <= n && m < a.M && b < a.nb) {
-      auto D = [&](int set) -> double2 {  // -( (n+1) eps_n c_{n-1} - n eps_{n+1} c_{n+1} )
-        const double e0 = (n + 1) * ev[i][0], e1 = n * ev[i][1];
-        const double2 cm = c[i][0][set], cp = c[i][2][set];
-        return make_double2(e1 * cp.x - e0 * cm.x, e1 * cp.y - e0 * cm.y);
-      };
-      if (OP == PACK_PLAIN) {
-        v0 = c[i][1][0];
-      } else if (OP == PACK_DIVLAMBDA) {
-        v0 = times_im(c[i][1][0], m);
-      } else if (OP == PACK_DIVMU) {
-        v0 = D(0);
-      } else if (OP == PACK_ALPHA) {
-        v0 = cscale(cadd(times_im(c[i][1][0], m), D(1)), 1.0 / a.radius);
-      } else {  // PACK_VORDIV: set 0 = U cos, set 1 = V cos
-        v0 = cscale(csub(times_im(c[i][1][1], m), D(0)), 1.0 / a.radius);
-        v1 = cscale(cadd(times_im(c[i][1][0], m), D(1)), 1.0 / a.radius);
-      }
-    }
+    if (m <= n && m < a.M && b < a.nb) pack_combine<OP>(c[i], n, m, ev[i][0], ev[i][1], a.radius, v0, v1);
     const double s = (m == 0) ? 1.0 : kSqrt2;
     out[0][0][mi][lane] = v0.x * s;
     out[0][1][mi][lane] = v0.y * s;
@@ -164,19 +99,6 @@ __global__ void __launch_bounds__(256) k_pack(SpecArgs a)
   }
 }
 
-// Which staged runs an unpack operator reads.  A run is (input, degree offset
-// dn = -1/0/+1, cos/sin part); runs are numbered in*6 + (dn+1)*2 + part.
-template <int OP>
-__host__ __device__ constexpr bool unpack_needs(int in, int dn)
-{
-  return OP == UNPACK_PLAIN || OP == UNPACK_GRADLAMBDA ? (in == 0 && dn == 0)
-       : OP == UNPACK_GRADMU                          ? (in == 0 && dn != 0)
-       : OP == UNPACK_HGRAD                           ? (in == 0)
-       : OP == UNPACK_ALPHA                           ? (in == 0 ? dn == 0 : dn != 0)
-                                                      : true;  // VORDIV2UV
-}
-template <int OP>
-__host__ __device__ constexpr int unpack_outputs() { return OP == UNPACK_VORDIV2UV || OP == UNPACK_HGRAD ? 2 : 1; }
 
 // A warp takes field-levels b0 + 8 i' + w with its lanes along the orders
 // (256-byte runs of the SPML rows), applies the operator there, and stages
@@ -230,50 +152,18 @@ __global__ void __launch_bounds__(256) k_unpack(SpecArgs a)
         if (w && o >= 0) x[q][in][r / 2][r & 1] = __ldg(w + o);
       }
   const bool mok = m <= n && m <= a.N && m < a.M;
-  double ep = 0.0, em = 0.0;  // R(x)_n = (n+2) eps_{n+1} x_{n+1} - (n-1) eps_n x_{n-1}
+  double ep = 0.0, em = 0.0;
   if (kEps && mok) {
     ep = (n + 2) * eps_at(a, m, n + 1);
     em = (n - 1) * eps_at(a, m, n);
   }
-  // -a^2/(k(k+1)) for the degrees n - 1, n, n + 1
-  double lap[3] = {0.0, 0.0, 0.0};
-  if constexpr (OP == UNPACK_VORDIV2UV) {
-    const double a2 = a.radius * a.radius;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      const double k = n + d - 1.0;
-      lap[d] = k >= 1.0 ? -a2 / (k * (k + 1.0)) : 0.0;
-    }
-  }
+  double lap[3];
+  lap_factors<OP>(n, a.radius, lap);
   const double s = (m == 0) ? 1.0 : kRSqrt2;
 #pragma unroll
   for (int q = 0; q < NQ; ++q) {
-    auto coef = [&](int in, int dn) { return make_double2(x[q][in][dn + 1][0] * s, x[q][in][dn + 1][1] * s); };
-    auto R = [&](int in, bool inv_lap) {
-      double2 xp = coef(in, 1), xm = coef(in, -1);
-      if (inv_lap) {
-        xp = cscale(xp, lap[2]);
-        xm = cscale(xm, lap[0]);
-      }
-      return make_double2(ep * xp.x - em * xm.x, ep * xp.y - em * xm.y);
-    };
     double2 v0, v1 = make_double2(0.0, 0.0);
-    if (OP == UNPACK_PLAIN) {
-      v0 = coef(0, 0);
-    } else if (OP == UNPACK_GRADLAMBDA) {
-      v0 = times_im(coef(0, 0), m);
-    } else if (OP == UNPACK_GRADMU) {
-      v0 = R(0, false);
-    } else if (OP == UNPACK_HGRAD) {
-      v0 = times_im(coef(0, 0), m);
-      v1 = R(0, false);
-    } else if (OP == UNPACK_ALPHA) {
-      v0 = cadd(times_im(coef(0, 0), m), R(NIN - 1, false));
-    } else {  // UNPACK_VORDIV2UV: input 0 = vor, 1 = div
-      const double2 psi = cscale(coef(0, 0), lap[1]), chi = cscale(coef(NIN - 1, 0), lap[1]);
-      v0 = csub(times_im(chi, m), R(0, true));
-      v1 = cadd(times_im(psi, m), R(NIN - 1, true));
-    }
+    unpack_combine<OP>(x[q], m, ep, em, lap, s, v0, v1);
     ws[0][lane][8 * q + warp] = v0.x;
     ws[1][lane][8 * q + warp] = v0.y;
     if constexpr (NOUT == 2) {
