@@ -19,6 +19,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import sys
 
 import numpy as np
 import numpy as _numpy  # SpmlUtil_Init's argument `np` shadows the usual alias
@@ -155,6 +156,15 @@ def launch_count() -> int:
     return int(load_library().sht_launch_count())
 
 
+def _torch():
+    return sys.modules["torch"]  # only reached with a torch tensor in hand
+
+
+def _raw_stream():
+    """Device index -> handle of torch's current stream (0 for the default one)."""
+    return _torch()._C._cuda_getCurrentRawStream
+
+
 def _is_torch_cuda(x) -> bool:
     return type(x).__module__.startswith("torch") and getattr(x, "is_cuda", False)
 
@@ -271,18 +281,19 @@ class SpmlUtil:
         return (s[0] if len(s) == 2 else 1), len(s) == 2
 
     def _set_torch_stream(self, x):
-        import torch
-        s = torch.cuda.current_stream(x.device)
-        _check(load_library().sht_set_stream(self._h, _VP(s.cuda_stream)), "set_stream")
+        # the raw handle: building a Stream object costs more than the call it is for
+        st = _lib.sht_set_stream(self._h, _raw_stream()(x.get_device()))
+        if st != SHT_OK:
+            _check(st, "set_stream")
 
     def _run(self, name, ins, out_kind, nout=1):
         """ins: list of inputs (same kind); out_kind: 'grid' | 'spec' | 'avr' | 'ya'."""
-        lib = load_library()
         x0 = ins[0]
-        nb, batched = (self._grid_shape(x0) if x0.shape[-1] == self.im and x0.ndim >= 2 and x0.shape[-2] == self.jm
+        shape = x0.shape
+        nb, batched = (self._grid_shape(x0) if shape[-1] == self.im and len(shape) >= 2 and shape[-2] == self.jm
                        else self._spec_shape(x0))
         for x in ins[1:]:  # None: an optional input left out (a null pointer)
-            if x is not None and tuple(x.shape) != tuple(x0.shape):
+            if x is not None and tuple(x.shape) != tuple(shape):
                 raise SpmlError(1, name, "input shapes differ")
         if out_kind == "grid":
             oshape = (nb, self.jm, self.im)
@@ -293,22 +304,25 @@ class SpmlUtil:
         else:
             oshape = (nb, self.jm)
         if _is_torch_cuda(x0):
-            import torch
+            f64 = _torch().float64
             ins = [None if x is None else x.contiguous() for x in ins]
-            if any(x is not None and x.dtype != torch.float64 for x in ins):
-                raise SpmlError(1, name, "device arrays must be float64")
-            outs = [torch.empty(oshape, dtype=torch.float64, device=x0.device) for _ in range(nout)]
+            for x in ins:
+                if x is not None and x.dtype != f64:
+                    raise SpmlError(1, name, "device arrays must be float64")
+            outs = [x0.new_empty(oshape) for _ in range(nout)]
             self._set_torch_stream(x0)
-            st = getattr(lib, name + "_dev")(self._h, *(_VP(None if x is None else x.data_ptr()) for x in ins), nb,
-                                             *(_VP(o.data_ptr()) for o in outs))
+            st = getattr(_lib, name + "_dev")(self._h, *[None if x is None else x.data_ptr() for x in ins], nb,
+                                              *[o.data_ptr() for o in outs])
         else:
+            lib = load_library()
             ins = [None if x is None else np.ascontiguousarray(x, dtype=np.float64) for x in ins]
             outs = [np.empty(oshape) for _ in range(nout)]
             st = getattr(lib, name)(self._h, *(_VP(None if x is None else x.ctypes.data) for x in ins), nb,
                                     *(_VP(o.ctypes.data) for o in outs))
-        _check(st, name)
+        if st != SHT_OK:
+            _check(st, name)
         if not batched:
-            outs = [o[0] if out_kind != "avr" else o[0] for o in outs]
+            outs = [o[0] for o in outs]
         return outs[0] if nout == 1 else tuple(outs)
 
     # ------------------------------------------------- transforms (a2 - a12)
