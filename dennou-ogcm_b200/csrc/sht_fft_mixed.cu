@@ -22,9 +22,12 @@
 // blocks per SM).  What it replaces, the direct sum over longitudes, is O(I N)
 // per row and bound by its FP64 products.  The T106 grid (320 x 160, 180
 // field-levels, 123 MB per direction): forward / inverse 0.730 / 1.289 ms ->
-// 0.031 / 0.044 ms, 4.0 / 2.8 TB/s; 192 x 96, 74 columns: 61 / 112 -> 6.9 / 9.2 us.
+// 0.031 / 0.037 ms, 4.0 / 3.3 TB/s; 192 x 96, 74 columns: 61 / 112 -> 6.9 / 7.1 us.
 #include "sht_fft_tile.cuh"
 #include "sht_fft_mixed.cuh"
+
+#include <algorithm>
+#include <type_traits>
 
 namespace sht {
 
@@ -219,9 +222,11 @@ __device__ __forceinline__ void with_radix(int r, F &&f)
   case 16: f(integral_constant<int, 16>()); break;
   default:
     if constexpr (MAXR > 16) {
+      if (r == 18) f(integral_constant<int, 18>());
+      if (r == 20) f(integral_constant<int, 20>());
+    }
+    if constexpr (MAXR > 20) {
       switch (r) {
-      case 18: f(integral_constant<int, 18>()); break;
-      case 20: f(integral_constant<int, 20>()); break;
       case 24: f(integral_constant<int, 24>()); break;
       case 25: f(integral_constant<int, 25>()); break;
       case 27: f(integral_constant<int, 27>()); break;
@@ -449,6 +454,223 @@ __global__ void __launch_bounds__(256, MAXR <= 16 ? 2 : 1) k_mix_inv(MixArgs a)
   }
 }
 
+// ------------------------------------------- mirrored pairs as one complex row
+// For I = R1 R2 itself (im up to 960 or so) the north and south row of a
+// mirrored pair are the real and imaginary part of one complex row of I points,
+// as in sht_fft_row.cu: both unpack from Z_m and Z_{I-m} without a twiddle, and
+// only the outputs m <= N and m >= I - N pass through shared memory.  The
+// inverse's Fourier runs of the next tile stream into their own buffer
+// (cp.async) while this one is transformed.
+struct PairShared {
+  double2 *stw, *buf, *runs;
+  unsigned short *pos;
+};
+
+// stw[k1 R2 + u] = W_I^{u k1}; pos[m]: the slot of order m (I - m below m = 0)
+template <bool INV>
+__device__ __forceinline__ PairShared pair_shared(const MixArgs &a)
+{
+  extern __shared__ __align__(16) double2 smem_mix[];
+  const int I = a.f.I, R1 = a.R1, R2 = a.R2;
+  PairShared s;
+  s.stw = smem_mix;
+  s.buf = smem_mix + I;
+  s.runs = s.buf + (a.RS << a.lgh);
+  s.pos = reinterpret_cast<unsigned short *>(s.runs + (INV ? (a.f.N + 1) * (2 << a.lgh) : 0));
+  for (int q = threadIdx.x; q < I; q += blockDim.x) {
+    const int t = (q % R2) * (q / R2);
+    const double2 w = __ldg(a.f.twI + (t < I / 2 ? t : t - I / 2));
+    s.stw[q] = t < I / 2 ? w : make_double2(-w.x, -w.y);
+    s.pos[q] = (unsigned short)(INV ? (q / R2) * a.S + q % R2 : (q % R1) * a.S + q / R1);
+  }
+  return s;
+}
+
+template <int MAXR, int MUL>
+__global__ void __launch_bounds__(256, MAXR <= 20 ? 2 : 1) k_mixpair_fwd(MixArgs a)
+{
+  const FftArgs &f = a.f;
+  const int I = f.I, R1 = a.R1, R2 = a.R2, S = a.S, RS = a.RS;
+  const int JTh = 1 << a.lgh, NT = blockDim.x, tid = threadIdx.x;
+  const PairShared sh = pair_shared<false>(a);
+  double2 *const buf = sh.buf;
+  __syncthreads();
+  const unsigned ntile = (unsigned)((f.JH + JTh - 1) >> a.lgh);
+  const unsigned ntot = (unsigned)f.ncol * ntile;
+  const long long IJ = (long long)I * f.J, mstride = (long long)f.ncolF * f.J;
+  const uint64_t keep = l2::keep_policy();
+  for (unsigned t0 = blockIdx.x; t0 < ntot; t0 += gridDim.x) {
+    // last column first, as in the power-of-two kernels
+    const unsigned t = ntot - 1 - t0, c2 = t / ntile;
+    const int h0 = (int)(t - c2 * ntile) << a.lgh;
+    const int col = f.mul_pair ? (int)(c2 >> 1) + (int)(c2 & 1) * f.nsplit : (int)c2;
+    const double *gb = f.gcol ? f.gcol[col]
+                     : (col < f.nsplit) ? f.g0 + (long long)col * IJ : f.g1 + (long long)(col - f.nsplit) * IJ;
+    const double *fb = MUL ? f.mul + (long long)(col % f.nmul) * IJ : nullptr;
+    const double *zb = (MUL && f.add0) ? (col < f.nsplit ? f.add0 + (long long)col * IJ
+                                                         : f.add1 + (long long)(col - f.nsplit) * IJ) : nullptr;
+    with_radix<MAXR>(R1, [&](auto rc) {
+      constexpr int R = decltype(rc)::value;
+      for (int idx = tid; idx < R2 << a.lgh; idx += NT) {
+        const int row = idx / R2, u = idx - row * R2;
+        const bool valid = h0 + row < f.JH;
+        const int jn = f.JH + (valid ? h0 + row : 0), js = f.J - 1 - jn;
+        const int on = jn * I + u, os = js * I + u;
+        double2 v[R];
+#pragma unroll
+        for (int n = 0; n < R; ++n)
+          v[n] = valid ? make_double2(__ldcs(gb + on + R2 * n), __ldcs(gb + os + R2 * n)) : make_double2(0.0, 0.0);
+        if (MUL && valid) {
+#pragma unroll
+          for (int n = 0; n < R; ++n) {
+            v[n].x *= __ldg(fb + on + R2 * n);
+            v[n].y *= __ldg(fb + os + R2 * n);
+          }
+          if (zb) {
+#pragma unroll
+            for (int n = 0; n < R; ++n) {
+              v[n].x += __ldg(zb + on + R2 * n);
+              v[n].y += __ldg(zb + os + R2 * n);
+            }
+          }
+        }
+        dft_nat<R, false>(v);
+        double2 *o = buf + row * RS + u;
+        o[0] = v[0];
+#pragma unroll
+        for (int k = 1; k < R; ++k) o[k * S] = cmul(v[k], sh.stw[k * R2 + u]);
+      }
+    });
+    __syncthreads();
+    with_radix<MAXR>(R2, [&](auto rc) {
+      constexpr int R = decltype(rc)::value;
+      for (int idx = tid; idx < R1 << a.lgh; idx += NT) {
+        const int row = idx / R1, k1 = idx - row * R1;
+        double2 *o = buf + row * RS + k1 * S;
+        double2 v[R];
+#pragma unroll
+        for (int n = 0; n < R; ++n) v[n] = o[n];
+        dft_nat<R, false>(v);
+#pragma unroll
+        for (int n = 0; n < R; ++n) {
+          const int m = k1 + R1 * n;
+          if (m <= f.N || m >= I - f.N) o[n] = v[n];
+        }
+      }
+    });
+    __syncthreads();
+    // Gs = X + Y and Ga = X - Y from U = Z_m + conj Z_{I-m}, V = Z_m - conj Z_{I-m}
+    double2 *Fb = f.F + (long long)(f.colF0 + col) * f.J + h0;
+    for (int idx = tid; idx < (f.N + 1) << a.lgh; idx += NT) {
+      const int m = idx >> a.lgh, i = idx & (JTh - 1);
+      if (h0 + i >= f.JH) continue;
+      const double sc = 0.5 * __ldg(f.rowscale + f.JH + h0 + i);  // the scales are symmetric in latitude
+      const double2 x = buf[i * RS + sh.pos[m]], y = buf[i * RS + sh.pos[m == 0 ? 0 : I - m]];
+      const double ux = x.x + y.x, uy = x.y - y.y, vx = x.x - y.x, vy = x.y + y.y;
+      l2::st_keep(Fb + m * mstride + i, make_double2((ux + vy) * sc, m == 0 ? 0.0 : (uy - vx) * sc), keep);
+      l2::st_keep(Fb + m * mstride + f.JH + i, make_double2((ux - vy) * sc, m == 0 ? 0.0 : (uy + vx) * sc), keep);
+    }
+    __syncthreads();  // the next tile reuses the buffer
+  }
+}
+
+template <int MAXR>
+__global__ void __launch_bounds__(256, MAXR <= 20 ? 2 : 1) k_mixpair_inv(MixArgs a)
+{
+  const FftArgs &f = a.f;
+  const int I = f.I, R1 = a.R1, R2 = a.R2, S = a.S, RS = a.RS;
+  const int JTh = 1 << a.lgh, MS = 2 * JTh, NT = blockDim.x, tid = threadIdx.x;
+  const PairShared sh = pair_shared<true>(a);
+  double2 *const buf = sh.buf, *const runs = sh.runs;
+  const unsigned ntile = (unsigned)((f.JH + JTh - 1) >> a.lgh);
+  const unsigned ntot = (unsigned)f.ncol * ntile;
+  const long long IJ = (long long)I * f.J, mstride = (long long)f.ncolF * f.J;
+  const bool drop = JTh * 16 % 128 == 0 && f.JH % JTh == 0;  // the runs are whole 128-byte lines
+  // runs[m MS + i] takes E, runs[m MS + JTh + i] O, of row pair h0 + i
+  auto issue = [&](unsigned t) {
+    const int col = (int)(t / ntile), h0 = (int)(t - (unsigned)col * ntile) << a.lgh;
+    const double2 *Fb = f.Fc + (long long)(f.colF0 + col) * f.J + h0;
+    for (int idx = tid; idx < (f.N + 1) << (a.lgh + 1); idx += NT) {
+      const int m = idx >> (a.lgh + 1), rr = idx & (MS - 1), i = rr & (JTh - 1);
+      const bool in = h0 + i < f.JH;
+      cp_async16(runs + idx, in ? Fb + m * mstride + (rr < JTh ? 0 : f.JH) + i : Fb, in);
+    }
+  };
+  unsigned t = blockIdx.x;
+  if (t < ntot) issue(t);
+  cp_async_commit();
+  for (; t < ntot; t += gridDim.x) {
+    const int col = (int)(t / ntile), h0 = (int)(t - (unsigned)col * ntile) << a.lgh;
+    const double2 *Fb = f.Fc + (long long)(f.colF0 + col) * f.J + h0;
+    cp_async_wait<0>();
+    __syncthreads();  // the runs (and the tables) are in; the row buffer is free
+    // Z_m = X + i Y and Z_{I-m} = conj X + i conj Y, X = E + O (north), Y = E - O
+    for (int idx = tid; idx < (f.N + 1) << a.lgh; idx += NT) {
+      const int m = idx >> a.lgh, i = idx & (JTh - 1);
+      const double2 e = runs[m * MS + i], o = runs[m * MS + JTh + i];
+      const double xr = e.x + o.x, yr = e.x - o.x;
+      const double xi = m == 0 ? 0.0 : e.y + o.y, yi = m == 0 ? 0.0 : e.y - o.y;
+      double2 *const z = buf + i * RS;
+      z[sh.pos[m]] = make_double2(xr - yi, xi + yr);
+      if (m > 0) z[sh.pos[I - m]] = make_double2(xr + yi, yr - xi);
+    }
+    __syncthreads();  // the runs are consumed, the rows complete
+    if (drop) {
+      // no later kernel reads these lines: drop them from L2 without a write-back
+      const int lpr = JTh * 16 / 128;
+      for (int q = tid; q < (f.N + 1) * 2 * lpr; q += NT) {
+        const int m = q / (2 * lpr), rest = q - m * 2 * lpr;
+        l2::discard_line(reinterpret_cast<const char *>(Fb + m * mstride + (rest < lpr ? 0 : f.JH)) + 128 * (rest % lpr));
+      }
+    }
+    if (t + gridDim.x < ntot) issue(t + gridDim.x);
+    cp_async_commit();
+    with_radix<MAXR>(R1, [&](auto rc) {
+      constexpr int R = decltype(rc)::value;
+      for (int idx = tid; idx < R2 << a.lgh; idx += NT) {
+        const int row = idx / R2, u = idx - row * R2;
+        double2 *o = buf + row * RS + u;
+        double2 v[R];
+#pragma unroll
+        for (int n = 0; n < R; ++n) {
+          const int m = R2 * n + u;
+          v[n] = make_double2(0.0, 0.0);
+          if (m <= f.N || m >= I - f.N) v[n] = o[n * S];
+        }
+        dft_nat<R, true>(v);
+        o[0] = v[0];
+#pragma unroll
+        for (int k = 1; k < R; ++k) o[k * S] = cmulc(v[k], sh.stw[k * R2 + u]);
+      }
+    });
+    __syncthreads();
+    double *dst = f.ocol ? f.ocol[col]
+                : (col < f.nsplit) ? f.o0 + (long long)col * IJ : f.o1 + (long long)(col - f.nsplit) * IJ;
+    with_radix<MAXR>(R2, [&](auto rc) {
+      constexpr int R = decltype(rc)::value;
+      for (int idx = tid; idx < R1 << a.lgh; idx += NT) {
+        const int row = idx / R1, k1 = idx - row * R1;
+        const double2 *o = buf + row * RS + k1 * S;
+        double2 v[R];
+#pragma unroll
+        for (int n = 0; n < R; ++n) v[n] = o[n];
+        dft_nat<R, true>(v);
+        if (h0 + row < f.JH) {
+          const int jn = f.JH + h0 + row, js = f.J - 1 - jn;
+          const double sc = __ldg(f.rowscale + jn);  // the scales are symmetric in latitude
+          double *const rn = dst + jn * I + k1, *const rs = dst + js * I + k1;
+#pragma unroll
+          for (int n = 0; n < R; ++n) {
+            rn[R1 * n] = v[n].x * sc;
+            rs[R1 * n] = v[n].y * sc;
+          }
+        }
+      }
+    });
+  }
+  cp_async_wait<0>();
+}
+
 constexpr int kRadices[] = {2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16, 18, 20, 24, 25, 27, 30, 32};
 
 // NC = R1 R2 over the radices above with the smallest larger one, which comes
@@ -469,35 +691,53 @@ bool radices(int NC, int *R1, int *R2)
 
 struct MixShape {
   MixArgs a;
+  bool pair;  // mirrored pairs as one complex row of I points; otherwise rows of I/2
   int threads;
   size_t smem;
 };
 
-bool mix_shape(int I, int N, MixShape *s)
+// Pairs in the inverse up to radix 20; otherwise rows of I/2 while their
+// radices stay at 16, then pairs.  Measured, rows / pairs, us: inverse im = 96,
+// 2000 field-levels 52 / 39, 240, 300 56 / 37, 320, 180 48 / 41, 480, 80 50 /
+// 62, 640, 60 125 / 72; forward 96 40 / 39, 192, 500 36 / 39, 320 38 / 42, 480
+// 39 / 67, 640 86 / 76.
+bool mix_shape(int I, int N, bool inverse, MixShape *s)
 {
   const int NC = I / 2;
   MixArgs &a = s->a;
-  if (!radices(NC, &a.R1, &a.R2)) return false;
+  int p1 = 0, p2 = 0, h1 = 0, h2 = 0;
+  const bool pair_ok = radices(I, &p1, &p2), half_ok = radices(NC, &h1, &h2);
+  if (!pair_ok && !half_ok) return false;
+  s->pair = pair_ok && (!half_ok || h1 > 16 || (inverse && p1 <= 20));
+  a.R1 = s->pair ? p1 : h1;
+  a.R2 = s->pair ? p2 : h2;
   a.S = a.R2 | 1;
   a.RS = (a.R1 * a.S) | 1;
+  auto bytes = [&](int lgh) {
+    if (s->pair)
+      return sizeof(double2) * (((size_t)a.RS << lgh) + I + (inverse ? (size_t)(N + 1) * (2 << lgh) : 0)) + sizeof(short) * ((size_t)I + 8);
+    return sizeof(double2) * ((size_t)(2 << lgh) * a.RS + 2 * (size_t)NC) + sizeof(short) * ((size_t)NC + 8);
+  };
   // eight row pairs per tile (128-byte Fourier runs) where at least three such
   // tiles share an SM, else four
-  auto bytes = [&](int lgh) { return sizeof(double2) * ((size_t)(2 << lgh) * a.RS + 2 * (size_t)NC) + sizeof(short) * ((size_t)NC + 8); };
   a.lgh = bytes(3) <= 75 * 1024 ? 3 : 2;
   s->smem = bytes(a.lgh);
-  // threads: the multiple of 32 with the least idle thread-time over the two
-  // passes (2 JT/2 R2 transforms of R1 points, then 2 JT/2 R1 of R2 points)
-  long long best = 0;
+  // threads: the most resident transforms per unit of pass time (rows R2
+  // transforms of R1 points, then rows R1 of R2 points; 128 or 255 registers a
+  // thread)
+  const int rows = s->pair ? 1 << a.lgh : 2 << a.lgh;
+  const int by_smem = (int)(227 * 1024 / (s->smem + 1024));
+  double best = 0.0;
   for (int nt = 96; nt <= 256; nt += 32) {
-    const int i1 = (2 << a.lgh) * a.R2, i2 = (2 << a.lgh) * a.R1;
-    const long long cost = (long long)nt * ((long long)((i1 + nt - 1) / nt) * a.R1 + (long long)((i2 + nt - 1) / nt) * a.R2);
-    if (best == 0 || cost <= best) {
-      best = cost;
+    const int i1 = rows * a.R2, i2 = rows * a.R1;
+    const int blocks = std::min(by_smem, (a.R1 <= 20 ? 512 : 256) / nt);
+    const double rate = blocks / (double)((i1 + nt - 1) / nt * a.R1 + (i2 + nt - 1) / nt * a.R2);
+    if (rate > best) {
+      best = rate;
       s->threads = nt;
     }
   }
-  (void)N;
-  return s->smem <= 227 * 1024;
+  return s->smem <= 227 * 1024 && best > 0.0;
 }
 
 }  // namespace
@@ -505,22 +745,34 @@ bool mix_shape(int I, int N, MixShape *s)
 bool fft_mixed_supported(int I, int N)
 {
   MixShape s{};
-  return I % 2 == 0 && mix_shape(I, N, &s);
+  return I % 2 == 0 && mix_shape(I, N, false, &s) && mix_shape(I, N, true, &s);
 }
 
 int run_fft_mixed(bool inverse, const sht_plan *p, const FftArgs &args, cudaStream_t s)
 {
   MixShape sh{};
-  if (!mix_shape(p->I, p->N, &sh)) { set_error("fft: longitude count without a two-pass factorisation"); return SHT_ERR_UNSUPPORTED_SIZE; }
+  if (!mix_shape(p->I, p->N, inverse, &sh)) { set_error("fft: longitude count without a two-pass factorisation"); return SHT_ERR_UNSUPPORTED_SIZE; }
   sh.a.f = args;
   const int JTh = 1 << sh.a.lgh;
   const long long ntiles = (long long)args.ncol * ((p->JH + JTh - 1) / JTh);
   if (ntiles <= 0) return SHT_OK;
   if (ntiles > 0x7fffffffLL) { set_error("fft: too many field-levels for one call"); return SHT_ERR_TOO_LARGE; }
-  const bool wide = sh.a.R1 > 16;
-  void (*kern)(MixArgs) = inverse ? (wide ? k_mix_inv<32> : k_mix_inv<16>)
-                        : args.mul ? (wide ? k_mix_fwd<32, 1> : k_mix_fwd<16, 1>)
-                                   : (wide ? k_mix_fwd<32, 0> : k_mix_fwd<16, 0>);
+  void (*kern)(MixArgs) = nullptr;
+  const int R = sh.a.R1;
+  if (sh.pair) {
+    auto pick = [&](auto mr) {
+      constexpr int MR = decltype(mr)::value;
+      kern = inverse ? k_mixpair_inv<MR> : args.mul ? k_mixpair_fwd<MR, 1> : k_mixpair_fwd<MR, 0>;
+    };
+    if (R <= 16) pick(std::integral_constant<int, 16>());
+    else if (R <= 20) pick(std::integral_constant<int, 20>());
+    else pick(std::integral_constant<int, 32>());
+  } else {
+    const bool wide = R > 16;
+    kern = inverse ? (wide ? k_mix_inv<32> : k_mix_inv<16>)
+         : args.mul ? (wide ? k_mix_fwd<32, 1> : k_mix_fwd<16, 1>)
+                    : (wide ? k_mix_fwd<32, 0> : k_mix_fwd<16, 0>);
+  }
   int occ = 0;
   cudaError_t e = kernel_setup((const void *)kern, sh.smem, sh.threads, &occ);
   if (e != cudaSuccess) return cuda_fail(e, "fft smem attribute");
