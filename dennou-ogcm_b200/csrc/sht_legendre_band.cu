@@ -33,16 +33,20 @@
 //     latitudes of one column (analysis), or of 8 columns of one degree
 //     (synthesis; lane n takes column n/2 + 4 (n mod 2) of the eight, which
 //     spreads each 8-lane phase over all banks).
-// Units are listed largest first and dealt out to the resident blocks forwards
-// and backwards in turn, which balances the triangular bands.
+// Units are listed largest first and dealt out to the SMs forwards and backwards
+// in turn, which balances the triangular bands; where units are long, the three
+// teams of an SM share its units.  Three independent blocks with equal shares
+// lose up to a quarter of the time there: the warp schedulers serve the oldest
+// first, and the youngest is left to finish alone (T170: the blocks of an SM
+// ended after 300, 325 and 420 thousand cycles).
 //
-// Bound: the FP64 tensor pipe from T170 up (72-76 % busy; the rest is padding
-// to 8-row tiles and the units' first and last stages), the Fourier array's
-// traffic and the units' latency below.  Measured against the kernels it
-// replaced (analysis / synthesis, us): T42, 3095 field-levels 52 / 48 -> 38 /
-// 36; T85, 480: 39.6 / 42.0 -> 31.5 / 31.5; 320 x 160 (T106), 180: 70 / 82 -> 27
-// / 25; T170, 720: 434 / 396 -> 221 / 215; T341, 240: 909 / 987 -> 506 / 508
-// (29 TF/s of the 37 executed).  Filling the stages with cp.async from the
+// Bound: the FP64 tensor pipe from T170 up (82-86 % of its rate with the padding
+// to 8-row tiles counted; the inner loop alone reaches 97 %), the Fourier
+// array's traffic and the units' latency below.  Measured against the kernels it
+// replaced (analysis / synthesis, us): T42, 3095 field-levels 52 / 48 -> 37 /
+// 35; T85, 480: 39.6 / 42.0 -> 30.7 / 30.7; 320 x 160 (T106), 180: 70 / 82 -> 27
+// / 25; T170, 720: 434 / 396 -> 207 / 195; T341, 240: 909 / 987 -> 483 / 475
+// (30.5 TF/s of the 37 executed).  Filling the stages with cp.async from the
 // consumer warps instead took 268 / 264 us at T170: their copy instructions
 // (up to ten per product) held the pipe at 61 %.
 #include "sht_internal.h"
@@ -76,9 +80,9 @@ struct BandArgs {
   int *err;           // host-mapped error word of the plan
 };
 
-// k-th unit of block b: the largest-first list is dealt out to the G resident
-// blocks forwards and backwards in turn, so that their shares differ by less
-// than one unit's work
+// k-th unit of block b: the largest-first list is dealt out to the G blocks
+// forwards and backwards in turn, so that their shares differ by less than one
+// unit's work
 __device__ __forceinline__ int unit_of(int k)
 {
   const int G = gridDim.x, b = blockIdx.x;
@@ -92,9 +96,17 @@ struct BandStage {
   static constexpr int BB = W * 8 * kKC * 16, AB = TM * 1024, BYTES = BB + AB;
 };
 
+// What a unit's first stage tells the consumers; col0 < 0: no more units.
+struct alignas(16) BandUnit {
+  BandItem item;
+  int col0, pad[3];
+};
+
+// Barriers and unit slots of one team; the block's unit counter and abort flag
 struct BandCtl {
   uint64_t *full, *empty;
-  int *abort_flag, *err;
+  BandUnit *unit;
+  int *taken, *abort_flag, *err;
 };
 
 // Waits for a phase, for at most two seconds of wall time: then the error word
@@ -137,30 +149,49 @@ __device__ __forceinline__ void tma_3d(void *dst, const CUtensorMap *map, int x,
       : "memory");
 }
 
-// The producer warp: every stage of the block's units in order.
-template <int W, int TM, int NS, bool INV>
+// A team's producer warp: every stage of the team's units in order, then a stage
+// that says there are no more.  The units come off the block's counter, so that
+// whichever team is ahead takes the next one; one is fetched ahead, since the
+// smallest units have a stage or two.
+template <int W, int TM, int NS, int TEAMS, bool INV>
 __device__ void band_produce(const BandArgs &a, const CUtensorMap *map, char *sm, const BandCtl &c)
 {
   using St = BandStage<W, TM>;
   const int lane = threadIdx.x & 31, CW = 1 << a.lgcw;
-  int u = unit_of(0), g = 0;  // g: stages issued so far
-  BandItem nxt = a.items[u / a.ncb];
-  for (int k = 1; u < a.nunits; ++k) {
+  int taken = 0;
+  auto take = [&] {
+    int k = taken++;
+    if constexpr (TEAMS > 1) {
+      if (lane == 0) k = atomicAdd(c.taken, 1);
+      k = __shfl_sync(0xffffffffu, k, 0);
+    }
+    return unit_of(k);
+  };
+  int g = 0;  // stages issued so far
+  bool ok = true;
+  int un = take();
+  BandItem nxt = a.items[un < a.nunits ? un / a.ncb : 0];
+  while (ok && un < a.nunits) {
+    const int u = un, col0 = (u % a.ncb) * (8 << a.lgcw);
     const BandItem it = nxt;
-    const int col0 = (u % a.ncb) * (8 << a.lgcw);
-    u = unit_of(k);
-    if (u < a.nunits) nxt = a.items[u / a.ncb];
+    un = take();
+    if (un < a.nunits) nxt = a.items[un / a.ncb];
     const int nrt = (it.cnt + 7) >> 3, nlt = (a.JH + 7) >> 3;
     const int nst = INV ? (nrt + 1) >> 1 : (nlt + 1) >> 1;
     const double *P = a.P + (INV ? it.blk + (long long)it.t0 * nrt : it.blk + it.t0) * 64;
     for (int st = 0; st < nst; ++st, ++g) {
       const int slot = g % NS;
-      if (g >= NS && !band_wait(c, c.empty + slot, ((g / NS) - 1) & 1)) goto drain;
+      if (g >= NS && !(ok = band_wait(c, c.empty + slot, ((g / NS) - 1) & 1))) break;
       char *B = sm + slot * St::BYTES, *A = B + St::BB;
       uint64_t *bar = c.full + slot;
       const int two = 2 * st + 1 < (INV ? nrt : nlt) ? 2 : 1;  // contraction tiles in this stage
-      if (lane == 0)
+      if (lane == 0) {
+        if (st == 0) {
+          c.unit[slot].item = it;
+          c.unit[slot].col0 = col0;
+        }
         tc::mbar_arrive_expect_tx(bar, (INV ? CW * 8 * kKC * 16 : two * CW * 1024) + two * it.tt * 512);
+      }
       __syncwarp();
       if constexpr (INV) {
         if (lane < CW) tma_3d(B + lane * 2048, map, 2 * (col0 + 8 * lane), it.row & 1, (it.row >> 1) + kKC * st, bar);
@@ -173,9 +204,14 @@ __device__ void band_produce(const BandArgs &a, const CUtensorMap *map, char *sm
       }
     }
   }
-  return;
-drain:
-  // leave only when this block's copies have landed in its shared memory
+  if (ok && (g < NS || band_wait(c, c.empty + g % NS, ((g / NS) - 1) & 1))) {
+    if (lane == 0) {
+      c.unit[g % NS].col0 = -1;
+      tc::mbar_arrive(c.full + g % NS);
+    }
+    return;
+  }
+  // aborted: leave only when the copies have landed in the block's shared memory
   for (int s = 0; s < NS && s < g; ++s) {
     const int last = g - 1 - (g - 1 - s) % NS;  // last stage issued to slot s
     const uint64_t t0 = tc::globaltimer_ns();
@@ -192,7 +228,7 @@ __device__ __forceinline__ bool band_fwd(const BandArgs &a, const char *sm, cons
                                          int col0)
 {
   using St = BandStage<W, TM>;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) % W;
   const int lgcw = SPLIT ? a.lgcw : __ffs(W) - 1;
   const int cg = warp & ((1 << lgcw) - 1), rw = SPLIT ? warp >> lgcw : 0;
   const int lgrw = SPLIT ? __ffs(W) - 1 - lgcw : 0, TT = SPLIT ? it.tt : T;
@@ -262,7 +298,7 @@ __device__ __forceinline__ bool band_inv(const BandArgs &a, const char *sm, cons
                                          int col0)
 {
   using St = BandStage<W, TM>;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) % W;
   const int lgcw = SPLIT ? a.lgcw : __ffs(W) - 1;
   const int cg = warp & ((1 << lgcw) - 1), rw = SPLIT ? warp >> lgcw : 0;
   const int lgrw = SPLIT ? __ffs(W) - 1 - lgcw : 0, TT = SPLIT ? it.tt : T;
@@ -343,42 +379,47 @@ __device__ __forceinline__ bool band_inv(const BandArgs &a, const char *sm, cons
   return true;
 }
 
-// The row tiles per warp (tt / RW rounded up) select the unrolled code.
-template <int W, int TM, int NS, int MINB, bool INV, bool SPLIT>
-__global__ void __launch_bounds__(32 * W + 32, MINB) k_leg_band(const __grid_constant__ CUtensorMap map, BandArgs a)
+// TEAMS teams of W consumer warps and a producer warp, each with its own ring of
+// stages and its own unit.  The row tiles per warp (tt / RW rounded
+// up) select the unrolled code.
+template <int W, int TM, int NS, int TEAMS, int MINB, bool INV, bool SPLIT>
+__global__ void __launch_bounds__(32 * (W + 1) * TEAMS, MINB) k_leg_band(const __grid_constant__ CUtensorMap map, BandArgs a)
 {
   extern __shared__ __align__(1024) char sm_band[];
-  uint64_t *bars = reinterpret_cast<uint64_t *>(sm_band + NS * BandStage<W, TM>::BYTES);
-  const BandCtl ctl{bars, bars + NS, reinterpret_cast<int *>(bars + 2 * NS), a.err};
+  constexpr int SLOTS = TEAMS * NS, STB = BandStage<W, TM>::BYTES;
+  BandUnit *units = reinterpret_cast<BandUnit *>(sm_band + SLOTS * STB);
+  uint64_t *bars = reinterpret_cast<uint64_t *>(units + SLOTS);
+  int *words = reinterpret_cast<int *>(bars + 2 * SLOTS);
   if (threadIdx.x == 0) {
-    for (int s = 0; s < NS; ++s) {
-      tc::mbar_init(ctl.full + s, 1);
-      tc::mbar_init(ctl.empty + s, W);
+    for (int s = 0; s < SLOTS; ++s) {
+      tc::mbar_init(bars + s, 1);
+      tc::mbar_init(bars + SLOTS + s, W);
     }
-    *ctl.abort_flag = 0;
+    words[0] = words[1] = 0;
     tc::mbar_fence_init();
   }
   __syncthreads();
-  int u = unit_of(0);
-  if (u >= a.nunits) return;
-  if (threadIdx.x >= 32 * W) {
-    band_produce<W, TM, NS, INV>(a, &map, sm_band, ctl);
+  // warps: the teams' consumers, then their producers
+  const int w = threadIdx.x >> 5, team = w < W * TEAMS ? w / W : w - W * TEAMS;
+  const BandCtl ctl{bars + team * NS, bars + SLOTS + team * NS, units + team * NS, words, words + 1, a.err};
+  char *const sm = sm_band + team * NS * STB;
+  if (w >= W * TEAMS) {
+    band_produce<W, TM, NS, TEAMS, INV>(a, &map, sm, ctl);
     return;
   }
-  BandItem nxt = a.items[u / a.ncb];
   const int lgrw = SPLIT ? __ffs(W) - 1 - a.lgcw : 0;
   int g = 0;  // stages consumed
-  for (int k = 1; u < a.nunits; ++k) {
-    const BandItem it = nxt;
-    const int col0 = (u % a.ncb) * (8 << a.lgcw);
-    u = unit_of(k);
-    if (u < a.nunits) nxt = a.items[u / a.ncb];
+  while (true) {
+    if (!band_wait(ctl, ctl.full + g % NS, (g / NS) & 1)) return;
+    const BandItem it = ctl.unit[g % NS].item;
+    const int col0 = ctl.unit[g % NS].col0;
+    if (col0 < 0) return;
     bool ok = true;
     auto go = [&](auto tc) {
       constexpr int T = decltype(tc)::value;
       if constexpr (T <= TM) {
-        if constexpr (INV) ok = band_inv<W, TM, T, NS, SPLIT>(a, sm_band, ctl, g, it, col0);
-        else ok = band_fwd<W, TM, T, NS, SPLIT>(a, sm_band, ctl, g, it, col0);
+        if constexpr (INV) ok = band_inv<W, TM, T, NS, SPLIT>(a, sm, ctl, g, it, col0);
+        else ok = band_fwd<W, TM, T, NS, SPLIT>(a, sm, ctl, g, it, col0);
       }
     };
     using std::integral_constant;
@@ -391,10 +432,7 @@ __global__ void __launch_bounds__(32 * W + 32, MINB) k_leg_band(const __grid_con
     case 6: go(integral_constant<int, 6>()); break;
     case 7: go(integral_constant<int, 7>()); break;
     case 8: go(integral_constant<int, 8>()); break;
-    case 9: go(integral_constant<int, 9>()); break;
-    case 10: go(integral_constant<int, 10>()); break;
-    case 11: go(integral_constant<int, 11>()); break;
-    default: break;
+      default: break;
     }
     if (!ok) return;
   }
@@ -426,12 +464,10 @@ int even_split(int tiles, int cap)
   return (tiles + nblk - 1) / nblk;
 }
 
-// Items of up to 8 tiles run three blocks per SM (128 registers), of up to 11
-// two blocks (160), re-reading the data operand less often.  11 pays for the
-// tallest outputs only (240 field-levels, analysis / synthesis: T341, 22 / 32
-// tiles, 531 / 524 -> 506 / 508 us); at 16 tiles the two are level (T170, 720:
-// 221 / 216 us), at 10 three blocks win (T106, 180: synthesis 27.6 -> 24.6 us).
-int item_cap(int tiles) { return tiles > 16 ? 11 : 8; }
+// 8 tiles of accumulators are what 128 registers hold; items of up to 11 (160
+// registers, two teams) re-read the data less often but took 506 / 508 us at
+// T341 where these take 483 / 475.
+constexpr int kItemCap = 8;
 
 }  // namespace
 
@@ -481,8 +517,8 @@ int plan_band_items(sht_plan *p, std::vector<long long> &boff, std::vector<BandI
       nb += (long long)nlt * ((count(m, par) + 7) / 8);
     }
   boff[2 * M] = nb;
-  p->band_tf = even_split(max_row_tiles(N), item_cap(max_row_tiles(N)));
-  p->band_ti = even_split(nlt, item_cap(nlt));
+  p->band_tf = even_split(max_row_tiles(N), kItemCap);
+  p->band_ti = even_split(nlt, kItemCap);
   std::vector<BandItem> inv;
   for (int m = 0; m < M; ++m)
     for (int par = 0; par < 2; ++par) {
@@ -565,10 +601,11 @@ int data_map(const sht_plan *p, const BandArgs &a, bool inv, const CUtensorMap *
   return SHT_OK;
 }
 
-template <int W, int TM, int NS, int MINB, bool INV>
+template <int W, int TM, int NS, int TEAMS, int MINB, bool INV>
 int run_band(const sht_plan *p, BandArgs a, cudaStream_t s)
 {
-  constexpr size_t smem = (size_t)NS * BandStage<W, TM>::BYTES + 16 * NS + 16;
+  constexpr size_t smem = (size_t)TEAMS * NS * (BandStage<W, TM>::BYTES + sizeof(BandUnit) + 16) + 16;
+  static_assert(MINB * (smem + 1024) <= 228 * 1024, "stages");
   // Columns per block: 8 W where the batch has that many.  A batch whose units
   // would leave block slots empty takes fewer (the warps then split the rows):
   // in the synthesis until the slots are filled (T85, 60 field-levels: 7.3 ->
@@ -578,7 +615,7 @@ int run_band(const sht_plan *p, BandArgs a, cudaStream_t s)
   int lg = 0;
   while ((1 << lg) < W && (8 << lg) < a.ncol) ++lg;
   auto units_at = [&](int l) { return (long long)items * ((a.ncol + (8 << l) - 1) / (8 << l)); };
-  const long long slots = (long long)MINB * grid_sms(p);
+  const long long slots = (long long)TEAMS * MINB * grid_sms(p);
   while (lg > 0 && (INV ? units_at(lg) < slots : units_at(lg - 1) <= slots)) --lg;
   a.lgcw = lg;
   a.ncb = (a.ncol + (8 << lg) - 1) / (8 << lg);
@@ -588,12 +625,12 @@ int run_band(const sht_plan *p, BandArgs a, cudaStream_t s)
   const CUtensorMap *map = nullptr;
   const int rc = data_map(p, a, INV, &map);
   if (rc) return rc;
-  auto kern = (1 << lg) == W ? k_leg_band<W, TM, NS, MINB, INV, false> : k_leg_band<W, TM, NS, MINB, INV, true>;
-  int occ = 0;
-  cudaError_t e = kernel_setup((const void *)kern, smem, 32 * W + 32, &occ);
+  auto kern = (1 << lg) == W ? k_leg_band<W, TM, NS, TEAMS, MINB, INV, false>
+                             : k_leg_band<W, TM, NS, TEAMS, MINB, INV, true>;
+  constexpr int threads = 32 * (W + 1) * TEAMS;
+  cudaError_t e = kernel_setup((const void *)kern, smem, threads);
   if (e != cudaSuccess) return cuda_fail(e, "legendre band smem attribute");
-  const long long gr = (long long)(occ < 1 ? 1 : occ) * grid_sms(p);
-  kern<<<(unsigned)std::min(units, gr), 32 * W + 32, smem, s>>>(*map, a);
+  kern<<<(unsigned)std::min<long long>(units, (long long)MINB * grid_sms(p)), threads, smem, s>>>(*map, a);
   count_launch();
   e = cudaGetLastError();
   return e == cudaSuccess ? SHT_OK : cuda_fail(e, "k_leg_band");
@@ -607,9 +644,14 @@ int launch_band(const sht_plan *p, BandArgs a, cudaStream_t s)
   a.J = p->J; a.JH = p->JH;
   a.err = p->err_word;
   const int tm = INV ? p->band_ti : p->band_tf;
-  if (tm <= 6) return run_band<4, 6, 4, 3, INV>(p, a, s);
-  if (tm <= 8) return run_band<4, 8, 4, 3, INV>(p, a, s);
-  return run_band<4, 11, 4, 2, INV>(p, a, s);
+  // One block of three teams, or three blocks of one.  The teams share the SM's
+  // units, which pays where a unit is long (analysis / synthesis, T170, 720:
+  // 221 / 215 -> 209 / 197 us, T341, 240: 506 / 508 -> 483 / 475); below, blocks
+  // that start and end apart are level or ahead (T85, 480: 32.8 / 30.7 either way,
+  // T42, 3095: 39.8 / 36.9 shared, 36.9 / 34.8 apart).
+  if (p->N > 127) return run_band<4, 8, 4, 3, 1, INV>(p, a, s);
+  if (tm <= 6) return run_band<4, 6, 4, 1, 3, INV>(p, a, s);
+  return run_band<4, 8, 4, 1, 3, INV>(p, a, s);
 }
 
 }  // namespace
