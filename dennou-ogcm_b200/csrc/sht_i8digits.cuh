@@ -160,24 +160,36 @@ __host__ __device__ inline double i2d(int32_t v)
   const uint32_t u = (uint32_t)v ^ 0x80000000u;
   return bits2d((int64_t)(((uint64_t)0x43300000u << 32) | u)) - 4503601774854144.0;  // 2^52 + 2^31
 }
-
-// sum_{L<8} A_L 256^(7-L) from the eight level sums.  For K <= 64 terms the
-// pairs (A_0, A_1), ..., (A_6, A_7) combine exactly in 32 bits (with |c_0| <= 4
-// in the data and <= 64 in the table: |A_0| <= 2^8 K, |A_1| <= 8704 K,
-// |A_L| <= (8704 + (L - 1) 2^14) K for L = 2..6, |A_7| <= (8192 + 6 2^14) K;
-// the largest pair, A_6 256 + A_7, stays below 1.5e9 at K = 64), so four
-// conversions suffice.
-__host__ __device__ inline double combine_levels(const int32_t (&a)[kLevels], bool k_le_64)
+// exact integer -> double for |v| < 2^51: one 64-bit integer and one FP64 operation
+__host__ __device__ inline double exact2d(int64_t v)
 {
-  static_assert(kLevels == 8, "level pairing below assumes eight levels");
-  if (k_le_64) {
-    const int32_t h1 = a[0] * 256 + a[1], h2 = a[2] * 256 + a[3], h3 = a[4] * 256 + a[5], h4 = a[6] * 256 + a[7];
-    return fma(fma(fma(i2d(h1), 65536.0, i2d(h2)), 65536.0, i2d(h3)), 65536.0, i2d(h4));
-  }
-  double d = i2d(a[0]);
-#pragma unroll
-  for (int L = 1; L < kLevels; ++L) d = fma(d, 256.0, i2d(a[L]));
-  return d;
+  return bits2d(v + 0x4338000000000000LL) - 6755399441055744.0;  // 1.5 2^52
+}
+
+// sum_{L<8} A_L 256^(7-L) from the eight level sums, rounded once.  With
+// |c_0| <= 4 in the data and <= 64 in the table, |A_0| <= 2^8 K, |A_1| <= 8704 K,
+// |A_L| <= (8704 + (L - 1) 2^14) K for L = 2..6 and |A_7| <= (8192 + 6 2^14) K.
+// So A_0 256 + A_1 fits 32 bits and the upper half (A_0..A_3) stays below 2^47
+// for K < 2^14; the lower half (A_4..A_7) stays below 2^51 for K <= kExactK.
+// The halves are added in integers: level by level in FP64 it took 23 FP64
+// operations per value (here five) and was most of the readout's arithmetic.
+constexpr int kExactK = 2048;
+__host__ __device__ inline double combine_levels(const int32_t (&a)[kLevels], bool exact)
+{
+  static_assert(kLevels == 8, "the halves below assume eight levels");
+  const int64_t hi = (int64_t)(a[0] * 256 + a[1]) * 65536 + ((int64_t)a[2] * 256 + a[3]);
+  const int64_t lo = (int64_t)a[4] * 16777216 + ((int64_t)a[5] * 65536 + ((int64_t)a[6] * 256 + a[7]));
+  return fma(exact2d(hi), 4294967296.0, exact ? exact2d(lo) : (double)lo);
+}
+
+// The same for K <= 64, where the four pairs (A_0, A_1), ... combine in 32 bits
+// (the largest, A_6 256 + A_7, stays below 1.5e9): no 64-bit products, three
+// roundings.
+constexpr int kPairK = 64;
+__host__ __device__ inline double combine_pairs(const int32_t (&a)[kLevels])
+{
+  const int32_t h1 = a[0] * 256 + a[1], h2 = a[2] * 256 + a[3], h3 = a[4] * 256 + a[5], h4 = a[6] * 256 + a[7];
+  return fma(fma(fma(i2d(h1), 65536.0, i2d(h2)), 65536.0, i2d(h3)), 65536.0, i2d(h4));
 }
 
 }  // namespace i8

@@ -22,7 +22,7 @@
 // accumulator set holds 8 x Npad <= 256 TMEM columns (two sets: a segment's
 // readout overlaps the next one's MMAs).
 //
-// Warp roles (one CTA of 448 threads per SM, persistent over a contiguous
+// Warp roles (one CTA of 448 or 512 threads per SM, persistent over a contiguous
 // slice of (band pair, 64-column tile, band, parity) sub-items):
 //   warp 0      table producer: bulk copies of the segment's table digits
 //   warp 1      TMEM allocation; one thread issues the MMAs and commits
@@ -32,20 +32,42 @@
 //   epilogue    TMEM level sums -> FP64 -> scaled outputs: 4 warps in the
 //               analysis, 8 in the synthesis (two per TMEM lane quadrant,
 //               alternate 4-row groups)
+//   exponents   (synthesis with the digit cache) the column exponents, from a
+//               pass over each sub-item's data ahead of the converters: 2 warps
 // Stages: two data-digit stages, two table stages, two accumulator sets and
 // four column-exponent slots, each with full/empty mbarriers.  Every wait is
 // bounded by 2 s of %globaltimer; a timeout sets the plan's device error word
 // and an abort flag that every role polls, and the CTA unwinds (waiting,
 // again bounded, for its own MMAs and copies) and frees its TMEM.
 //
-// A sub-item's data are converted once per group of two output segments
-// (once in all at T85 and below), K chunk by K chunk; when K spans several
-// chunks, the column exponents come from a first pass over all of them.
+// A sub-item's data are converted once, K chunk by K chunk; sub-items with more
+// than two output segments keep the digits for their later groups of two
+// segments (stage fills, below).  When K spans several chunks, the column
+// exponents come from a first pass over all of them.
+//
+// What bounds it, from clock readings per role (T341, 240 field-levels): the MMA
+// thread, whose 3900 MMAs of 74 cycles at least (measured alone: N/2 cycles, the
+// integer rate of the tensor pipe) take 100 to 130 with converters, copies and
+// readout on the same shared memory and TMEM; it waits a quarter of the time for the
+// readout (synthesis) or the converters (analysis).  Tensor pipe 19 % before, 23 %
+// now.  Contraction, synthesis / analysis, in us:
+//                        T85, 480    T170, 720    T341, 240    T341, 960
+//   before                83 / 62    471 / 404    840 / 764   3095 / 2756
+//   now                   73 / 56    408 / 323    633 / 652   2456 / 2379
+// Of that, at T341, synthesis / analysis: unconditional load batches, the cache
+// written by bulk copies instead of the converters' stores, exponents from their
+// own warps (synthesis) 840 -> 704 / 764 -> 735; stages kept from group to group
+// 680 / 709; level sums added as integers and whole-sector stores 637 / 709;
+// 32-byte loads 633 / 652.  Measured and not kept: exponent warps in the analysis
+// (T170 404 -> 477 us, its runs are read faster by eight warps), a coalesced
+// exponent pass there (T170 323 -> 342), two groups of converters on one stage
+// each (704 -> 781), polling without the suspend hint (no change).
 #include "sht_internal.h"
 #include "sht_tc.cuh"
 #include "sht_i8digits.cuh"
 #include "sht_l2.cuh"
 
+#include <type_traits>
 #include <vector>
 
 namespace sht {
@@ -73,20 +95,25 @@ struct Roles {
   static constexpr int kConv0 = 2, kEpi0 = kConv0 + kConvW;
   // values per thread in flight in the column-exponent pass over a sub-item's
   // other K chunks: 16 in the synthesis (strided coefficient rows), 4 in the
-  // analysis (contiguous Fourier runs; 16 measured slower at T341)
+  // analysis (contiguous Fourier runs; 16 measured slower at T170 and level at T341)
   static constexpr int kPreBatch = INV ? 16 : 4;
-  static constexpr int kThreads = 32 * (kEpi0 + kEpiW);
+  static constexpr int kScan0 = kEpi0 + kEpiW;  // the exponent warps
 };
-constexpr int kThreads = 448;
-static_assert(Roles<false>::kThreads == kThreads && Roles<true>::kThreads == kThreads, "block size");
+constexpr int kScanW = 2;
+static_assert(Roles<false>::kScan0 == 14 && Roles<true>::kScan0 == 14, "block size");
+// the synthesis with the digit cache takes its column exponents from two warps
+// of their own (a 512-thread block still has 128 registers per thread)
+constexpr bool scan_of(bool inv, bool cache) { return inv && cache; }
+constexpr int threads_of(bool scan) { return 32 * (14 + (scan ? kScanW : 0)); }
 constexpr int kSlots = 4;                            // column-exponent slots
+constexpr int kAhead = 1;                            // sub-items the exponent warps run ahead (1 to 3 level)
 constexpr uint64_t kWaitLimit = 2000000000ull;       // 2 s per bounded wait
 static_assert(kLevels * kSeg <= kSetCols && 2 * kSetCols <= 512, "TMEM columns");
 
 // barrier indices
 enum : int {
   B_PFULL = 0, B_PEMPTY = 2, B_DFULL = 4, B_DEMPTY = 6, B_AFULL = 8, B_AEMPTY = 10,
-  B_EFULL = 12, B_EEMPTY = 16, B_DONE = 20, B_CFULL = 21, B_SREADY = 23, B_COUNT = 25
+  B_EFULL = 12, B_EEMPTY = 16, B_DONE = 20, B_CFULL = 21, B_SREADY = 23, B_CEMPTY = 24, B_COUNT = 26
 };
 
 __host__ __device__ inline int rows_of_parity(int N, int m, int p)
@@ -111,7 +138,7 @@ struct I8Tables {
   long long *toff[2] = {nullptr, nullptr};   // byte offset per (m, p)
   double *tfac[2] = {nullptr, nullptr};      // row scale factors 2^(e_row - kShift)
   int *teoff[2] = {nullptr, nullptr};        // first row exponent per (m, p)
-  uint8_t *scr[2] = {nullptr, nullptr};      // digit cache: per CTA, two slots of the chunks of one sub-item
+  uint8_t *scr[2] = {nullptr, nullptr};      // digit cache: per CTA, the chunks of one sub-item
   long long scr_cta[2] = {0, 0};             // its bytes per CTA
   int *d_err = nullptr;                      // device error word
 };
@@ -173,7 +200,7 @@ struct I8Args {
   int ntiles, nsub, per_cta;
   int *err;
   uint8_t *scr;        // digit cache (null when no sub-item has more than two segments)
-  long long scr_cta;   // bytes of it per CTA: two slots of nchmax data stages
+  long long scr_cta;   // bytes of it per CTA: nchmax data stages
 };
 
 // Shared-memory copies of the small lookup tables (band pairs, internal row
@@ -196,11 +223,13 @@ __host__ __device__ inline size_t lut_bytes(int N, int npairs)
 struct Unit {
   int g;                  // sub-item: item g / 4, band/parity g % 4
   int m, p, Rp, K, nrow, nseg, nch;
-  int seg, ch;            // first segment of this unit's group, K chunk
+  int seg, ch;            // first segment of this unit's group, position of its chunk in the group
+  int chunk, fill;        // K chunk; number of its stage fill within the sub-item
   int col0;
   int sub_count;          // sub-items this CTA began before this one
   int seg_base;           // segments this CTA began before this sub-item
-  int csub;               // sub-items with more than two segments this CTA began before this one
+  int csub;               // sub-items that use the digit cache this CTA began before this one
+  int fill_base;          // stage fills of this CTA's earlier sub-items
   int rowoff, teoff;      // internal row of degree m, first row factor of (m, p)
   long long toff;         // table bytes of (m, p)
 };
@@ -228,7 +257,7 @@ __device__ __forceinline__ bool setup_sub(const I8Args &a, const Lut &t, int g, 
   u.nseg = nseg_of(u.nrow);
   u.nch = (u.K + kKC - 1) / kKC;
   u.seg = 0;
-  u.ch = 0;
+  u.ch = u.chunk = u.fill = 0;
   u.col0 = tile * (kM / 2);
   u.rowoff = t.rowoff[u.m];
   u.toff = t.toff[2 * u.m + u.p];
@@ -244,36 +273,74 @@ __device__ __forceinline__ bool first_unit(const I8Args &a, const Lut &t, int g0
       u.sub_count = 0;
       u.seg_base = 0;
       u.csub = 0;
+      u.fill_base = 0;
       return true;
     }
   return false;
 }
 
-template <bool INV>
+// Stage fills.  A sub-item with more than two output segments passes over its
+// K chunks once per group of two segments.  The two data stages still hold the
+// last two chunks of a group when the next group begins, so that group starts
+// with these two and goes on cyclically: fill i of a sub-item holds chunk i mod
+// nch, group g works on the nch fills from g (nch - 2) on (all groups on fill 0
+// if nch = 1), and nch - 2 fills per group are new.  The order of the chunks
+// does not matter, the level sums are exact integers.
+//
+// The first nch fills are converted.  Later ones come from the digit cache: the
+// MMA thread bulk-copies the converted stages that are needed again to the
+// CTA's cache, and the producer copies them back.  The MMA thread waits for
+// every copy back before it reaches the next sub-item's first stage, so one
+// sub-item's worth of cache is enough.
+__device__ __forceinline__ bool uses_cache(const Unit &u) { return u.nseg > 2 && u.nch > 2; }
+
+template <bool INV, bool CACHE>
 __device__ __forceinline__ bool next_unit(const I8Args &a, const Lut &t, int g1, Unit &u)
 {
-  if (++u.ch < u.nch) return true;
+  if (++u.ch < u.nch) {
+    ++u.fill;
+    if (++u.chunk == u.nch && CACHE) u.chunk = 0;
+    return true;
+  }
   u.ch = 0;
-  if ((u.seg += 2) < u.nseg) return true;
-  const int sc = u.sub_count + 1, sb = u.seg_base + u.nseg, cs = u.csub + (u.nseg > 2 ? 1 : 0);
+  if (CACHE && (u.seg += 2) < u.nseg) {  // without the cache no sub-item has more than one group
+    if (u.nch > 1) {
+      --u.fill;
+      u.chunk = (u.chunk == 0 ? u.nch : u.chunk) - 1;
+    }
+    return true;
+  }
+  const int sc = u.sub_count + 1, sb = u.seg_base + u.nseg, cs = u.csub + (CACHE && uses_cache(u) ? 1 : 0);
+  const int fb = u.fill_base + u.fill + 1;
   for (int g = u.g + 1; g < g1; ++g)
     if (setup_sub<INV>(a, t, g, u)) {
       u.sub_count = sc;
       u.seg_base = sb;
       u.csub = cs;
+      u.fill_base = fb;
       return true;
     }
   return false;
 }
 
-// Digit cache: a sub-item with more than two output segments is converted by
-// the converters once, in its first segment group, which also writes the
-// digit stages to the CTA's cache slot; its later groups take the stages from
-// there by bulk copy.
-__device__ __forceinline__ bool unit_cached(const Unit &u) { return u.nseg > 2 && u.seg >= 2; }
+__device__ __forceinline__ bool new_fill(const Unit &u) { return u.seg == 0 || u.ch >= 2; }
+__device__ __forceinline__ bool last_use(const Unit &u) { return u.seg + 2 >= u.nseg || u.ch < u.nch - 2; }
+// The release of a stage goes to the role that fills it next, the producer
+// (true) or the converters: each role then waits for every phase of its own
+// barriers in turn, which a parity wait needs (it only tells the last two apart).
+__device__ __forceinline__ bool next_from_cache(const Unit &u)
+{
+  const int total = u.nch + (uses_cache(u) ? ((u.nseg + 1) / 2 - 1) * (u.nch - 2) : 0);
+  return u.fill + 2 >= u.nch && u.fill + 2 < total;
+}
+// converted fills that a later group copies back
+__device__ __forceinline__ bool to_cache(const Unit &u)
+{
+  return uses_cache(u) && u.seg == 0 && u.chunk < ((u.nseg + 1) / 2 - 1) * (u.nch - 2);
+}
 __device__ __forceinline__ uint8_t *cache_stage(const I8Args &a, const Unit &u)
 {
-  return a.scr + blockIdx.x * a.scr_cta + (u.csub & 1) * (a.scr_cta / 2) + (long long)u.ch * kStageA;
+  return a.scr + blockIdx.x * a.scr_cta + (long long)u.chunk * kStageA;
 }
 
 struct Ctl {
@@ -313,38 +380,43 @@ __device__ __forceinline__ bool warp_wait(const Ctl &c, int b, uint32_t parity)
 
 // No memory clobber: nothing in the kernel reads these outputs, and the
 // compiler stays free to overlap the stores with the next rows' arithmetic.
-__device__ __forceinline__ void st_keep_f64(double *ptr, double v, uint64_t policy)
+__device__ __forceinline__ void st_keep2(double2 *ptr, double2 v, uint64_t policy)
 {
-  asm volatile("st.global.L2::cache_hint.f64 [%0], %1, %2;\n" ::"l"(ptr), "d"(v), "l"(policy));
+  asm volatile("st.global.L2::cache_hint.v2.f64 [%0], {%1, %2}, %3;\n" ::"l"(ptr), "d"(v.x), "d"(v.y), "l"(policy));
 }
 
 // Four rows of one segment: level sums -> FP64 results, computed branch-free
 // (independent chains the scheduler can interleave), then stored.
-template <bool INV, bool FAST>
+template <bool INV, bool PAIRS>
 __device__ __forceinline__ void epilogue_rows(const I8Args &a, const Unit &u, int row0, int col, bool cv, int part,
                                               const uint32_t (&r)[kLevels][4], const double (&fr)[4], double fcol,
                                               uint64_t keep)
 {
+  const bool exact = u.K <= i8::kExactK;
   double v[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     int32_t lv[kLevels];
 #pragma unroll
     for (int L = 0; L < kLevels; ++L) lv[L] = (int32_t)r[L][i];
-    v[i] = i8::combine_levels(lv, FAST) * fcol * fr[i];
+    v[i] = (PAIRS ? i8::combine_pairs(lv) : i8::combine_levels(lv, exact)) * fcol * fr[i];
   }
-  if (!cv) return;
   if (!INV) {
+    if (!cv) return;
     double *dst = reinterpret_cast<double *>(a.S + ((long long)u.rowoff + u.p + 2 * row0) * a.ncol + col) + part;
     const long long step = 4 * (long long)a.ncol;  // two internal rows (one parity) per output row, in doubles
 #pragma unroll
     for (int i = 0; i < 4; ++i)
       if (row0 + i < u.nrow) dst[i * step] = v[i];
   } else {
-    double *dst = reinterpret_cast<double *>(a.Fo + ((long long)u.m * a.ncol + col) * a.J + u.p * a.JH + row0) + part;
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-      if (row0 + i < u.nrow) st_keep_f64(dst + 2 * i, v[i], keep);
+    // the real and imaginary lanes of a column trade values, so that they store
+    // one complex row each (rows part and 2 + part) and fill whole sectors
+    const double e0 = __shfl_xor_sync(0xffffffffu, part ? v[0] : v[1], 1);
+    const double e1 = __shfl_xor_sync(0xffffffffu, part ? v[2] : v[3], 1);
+    if (!cv) return;
+    double2 *dst = a.Fo + ((long long)u.m * a.ncol + col) * a.J + u.p * a.JH + row0 + part;
+    if (row0 + part < u.nrow) st_keep2(dst, part ? make_double2(e0, v[1]) : make_double2(v[0], e0), keep);
+    if (row0 + part + 2 < u.nrow) st_keep2(dst + 2, part ? make_double2(e1, v[3]) : make_double2(v[2], e1), keep);
   }
 }
 
@@ -354,14 +426,14 @@ template <bool INV, bool CACHE>
 __device__ void role_producer(const I8Args &a, const Ctl &c, unsigned char *Ps, unsigned char *As, const Lut &t, Unit u,
                               bool have, int g1)
 {
-  int k = 0, nc[2] = {0, 0};
-  int cpend[2] = {-1, -1};  // phase parity of the last cache copy into each data stage
-  for (; have; have = next_unit<INV>(a, t, g1, u), ++k) {
+  int k = 0;
+  uint32_t cany = 0, cpar = 0;  // per data stage: any cache copy issued, and the parity of its next one
+  for (; have; have = next_unit<INV, CACHE>(a, t, g1, u), ++k) {
     const int st = k & 1;
     if (k >= 2 && !wait_ph(c, B_PEMPTY + st, ((k >> 1) - 1) & 1)) break;
     const int s0 = u.seg, s1 = min(u.seg + 2, u.nseg);
     const int npt = npad_total(u.nrow);
-    const uint8_t *src = a.tab + u.toff + (long long)u.ch * kDigitsTable * kKC * npt +
+    const uint8_t *src = a.tab + u.toff + (long long)u.chunk * kDigitsTable * kKC * npt +
                          (long long)s0 * kDigitsTable * kKC * kSeg;
     uint32_t bytes = 0;
     for (int s = s0; s < s1; ++s) bytes += kDigitsTable * kKC * seg_npad(u.nrow, s);
@@ -372,38 +444,47 @@ __device__ void role_producer(const I8Args &a, const Ctl &c, unsigned char *Ps, 
       tc::bulk_g2s(Ps + st * kStageP + off, src + off, b, c.bar + B_PFULL + st);
       off += b;
     }
-    if (CACHE && unit_cached(u)) {
-      // the data digits of a later segment group: the converters wrote them to
-      // the cache slot in the sub-item's first group; the stage is free once
-      // the MMAs of unit k - 2 are done
-      if (u.seg == 2 && u.ch == 0 && !wait_ph(c, B_SREADY + (u.csub & 1), (u.csub >> 1) & 1)) break;
-      if (k >= 2 && !wait_ph(c, B_DEMPTY + st, ((k >> 1) - 1) & 1)) break;
-      tc::mbar_arrive_expect_tx(c.bar + B_CFULL + st, kStageA);
-      tc::bulk_g2s(As + st * kStageA, cache_stage(a, u), kStageA, c.bar + B_CFULL + st);
-      cpend[st] = nc[st] & 1;
-      ++nc[st];
+    if (CACHE && u.seg > 0 && new_fill(u)) {
+      // from the cache, once the sub-item's first group is in it
+      const int ds = (u.fill_base + u.fill) & 1;
+      if (u.fill == u.nch) {
+        if (!wait_ph(c, B_SREADY, u.csub & 1)) break;
+        tc::fence_proxy_async_global();
+      }
+      if (!wait_ph(c, B_CEMPTY + ds, (cpar >> ds) & 1)) break;
+      tc::mbar_arrive_expect_tx(c.bar + B_CFULL + ds, kStageA);
+      tc::bulk_g2s(As + ds * kStageA, cache_stage(a, u), kStageA, c.bar + B_CFULL + ds);
+      cany |= 1u << ds;
+      cpar ^= 1u << ds;
     }
   }
   // copies issued but never consumed (after an abort) must land before the CTA exits
   for (int j = (k >= 2 ? k - 2 : 0); j < k; ++j) wait_ph(Ctl{c.bar, c.abort_flag, c.err}, B_PFULL + (j & 1), (j >> 1) & 1);
   for (int st = 0; st < 2; ++st)
-    if (cpend[st] >= 0) wait_ph(c, B_CFULL + st, (uint32_t)cpend[st]);
+    if (cany >> st & 1) wait_ph(c, B_CFULL + st, ~(cpar >> st) & 1);
 }
 
 template <bool INV, bool CACHE>
 __device__ void role_mma(const I8Args &a, const Ctl &c, uint32_t As, uint32_t Ps, uint32_t tbase, const Lut &t, Unit u, bool have, int g1)
 {
-  int k = 0, nd[2] = {0, 0}, nc[2] = {0, 0};
-  for (; have; have = next_unit<INV>(a, t, g1, u), ++k) {
+  int k = 0;
+  uint32_t dpar = 0, cpar = 0;  // parity of each data stage's next phase, converted and copied
+  for (; have; have = next_unit<INV, CACHE>(a, t, g1, u), ++k) {
     const int st = k & 1;
     if (!wait_ph(c, B_PFULL + st, (k >> 1) & 1)) break;
-    // the data stage comes from the converters or, for a cached unit, from
-    // the producer's copy of the digit cache
-    if ((CACHE && unit_cached(u)) ? !wait_ph(c, B_CFULL + st, nc[st]++ & 1) : !wait_ph(c, B_DFULL + st, nd[st]++ & 1))
-      break;
+    const int ds = (u.fill_base + u.fill) & 1;
+    if (!CACHE || new_fill(u)) {
+      // from the converters, or by the producer's copy from the cache
+      const bool cached = CACHE && u.seg > 0;
+      if (!wait_ph(c, (cached ? B_CFULL : B_DFULL) + ds, ((cached ? cpar : dpar) >> ds) & 1)) break;
+      if (cached) cpar ^= 1u << ds;
+      else dpar ^= 1u << ds;
+    }
+    const bool keep = CACHE && to_cache(u);
+    if (keep) tc::bulk_s2g(cache_stage(a, u), As + ds * kStageA, kStageA);
     tc::fence_after();
     const int s0 = u.seg, s1 = min(u.seg + 2, u.nseg);
-    const int kvalid = min(kKC, u.K - u.ch * kKC);
+    const int kvalid = min(kKC, u.K - u.chunk * kKC);
     const int nks = (kvalid + 31) / 32;
     uint32_t pb = Ps + st * kStageP;
     bool ok = true;
@@ -416,71 +497,92 @@ __device__ void role_mma(const I8Args &a, const Ctl &c, uint32_t As, uint32_t Ps
         tc::fence_after();
       }
       const uint32_t d0 = tbase + (uint32_t)(set * kSetCols);
-      // descriptors built once; the start address (bits 0..13, in 16-byte
-      // units, below 256 KB of shared memory) then steps by plain adds
-      const uint64_t ad0 = tc::smem_desc(As + st * kStageA, 128, 512);
+      // Segments have 32 or 16 padded rows; with that a constant, an MMA costs
+      // two adds to the descriptors' low words (start address, in 16-byte units)
+      // and no other arithmetic.
+      const uint64_t ad0 = tc::smem_desc(As + ds * kStageA, 128, 512);
       const uint64_t bd0 = tc::smem_desc(pb, 128, 512);
-      const uint32_t id0 = tc::idesc_s8_s32(kM, 0);
-      // MMA of data digit sd against table digits [t0, t0 + nt): level sums
-      // L = sd + t go to accumulator columns from (sd + t0) npad on
-      auto mma = [&](int ks, int sd, int t0, int nt, uint32_t acc) {
-        const uint64_t ad = ad0 + (uint64_t)((sd * kTileA + ks * 256) >> 4);
-        const uint64_t bd = bd0 + (uint64_t)((t0 * npad * kKC + ks * 256) >> 4);
-        tc::mma_s8(d0 + (uint32_t)((sd + t0) * npad), ad, bd, id0 | ((uint32_t)(nt * npad) >> 3) << 17, acc);
-      };
-      static_assert(kLevels == kDigitsTable + 1, "data digits 0 and 1 pair with every table digit");
-      for (int ks = 0; ks < nks; ++ks) {
-        if (u.ch == 0 && ks == 0) {
-          // the segment's first K step initialises every level exactly once:
-          // digit 1 against t = 0..6 sets levels 1..7, digit 0 against t = 0
-          // sets level 0, and digit 0 against t = 1..6 adds to levels 1..6
-          mma(ks, 1, 0, kDigitsTable, 0u);
-          mma(ks, 0, 0, 1, 0u);
-          mma(ks, 0, 1, kDigitsTable - 1, 1u);
-        } else {
-          mma(ks, 0, 0, kDigitsTable, 1u);
-          mma(ks, 1, 0, kDigitsTable, 1u);
-        }
+      auto issue = [&](auto np) {
+        constexpr int NP = decltype(np)::value;
+        constexpr uint32_t id0 = tc::idesc_s8_s32(kM, 0);
+        for (int ks = 0; ks < nks; ++ks) {
+          const uint32_t al = (uint32_t)ad0 + 16 * ks, bl = (uint32_t)bd0 + 16 * ks;
+          // data digit sd against table digits [t0, t0 + nt): level sums
+          // L = sd + t go to accumulator columns from (sd + t0) NP on
+          auto mma = [&](int sd, int t0, int nt, uint32_t acc) {
+            const uint64_t ad = (ad0 & ~0xFFFFFFFFull) | (al + (uint32_t)(sd * kTileA >> 4));
+            const uint64_t bd = (bd0 & ~0xFFFFFFFFull) | (bl + (uint32_t)(t0 * NP * kKC >> 4));
+            tc::mma_s8(d0 + (uint32_t)((sd + t0) * NP), ad, bd, id0 | ((uint32_t)(nt * NP) >> 3) << 17, acc);
+          };
+          static_assert(kLevels == kDigitsTable + 1, "data digits 0 and 1 pair with every table digit");
+          if (u.ch == 0 && ks == 0) {
+            // the segment's first K step initialises every level exactly once:
+            // digit 1 against t = 0..6 sets levels 1..7, digit 0 against t = 0
+            // sets level 0, and digit 0 against t = 1..6 adds to levels 1..6
+            mma(1, 0, kDigitsTable, 0u);
+            mma(0, 0, 1, 0u);
+            mma(0, 1, kDigitsTable - 1, 1u);
+          } else {
+            mma(0, 0, kDigitsTable, 1u);
+            mma(1, 0, kDigitsTable, 1u);
+          }
 #pragma unroll
-        for (int sd = 2; sd < kDigitsData; ++sd) mma(ks, sd, 0, kLevels - sd, 1u);  // t < 8 - sd
-      }
+          for (int sd = 2; sd < kDigitsData; ++sd) mma(sd, 0, kLevels - sd, 1u);  // t < 8 - sd
+        }
+      };
+      if (npad == 32) issue(std::integral_constant<int, 32>{});
+      else issue(std::integral_constant<int, 16>{});
       if (u.ch == u.nch - 1) tc::mma_commit(c.bar + B_AFULL + set);
       pb += kDigitsTable * kKC * npad;
     }
     if (!ok) break;
-    tc::mma_commit(c.bar + B_DEMPTY + st);
+    if (keep) tc::bulk_wait_read();  // done behind the MMAs' issue
+    if (!CACHE || last_use(u)) tc::mma_commit(c.bar + (CACHE && next_from_cache(u) ? B_CEMPTY : B_DEMPTY) + ds);
     tc::mma_commit(c.bar + B_PEMPTY + st);
+    if (CACHE && uses_cache(u) && u.seg == 0 && u.ch == u.nch - 1) {
+      tc::bulk_wait();
+      tc::fence_proxy_async_global();
+      tc::mbar_arrive(c.bar + B_SREADY);
+    }
   }
+  if (CACHE) tc::bulk_wait();
   tc::mma_commit(c.bar + B_DONE);
 }
 
-// Load NV consecutive K values (k0 + i) of this thread's complex column.
-template <bool INV, int NV>
-__device__ __forceinline__ void loadn(const I8Args &a, const Unit &u, int col, bool cv, int k0, double2 (&x)[NV])
+__device__ __forceinline__ void ldg32(const double2 *p, double2 &x, double2 &y)
 {
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];\n" : "=d"(x.x), "=d"(x.y), "=d"(y.x), "=d"(y.y) : "l"(p));
+}
+// Load NV consecutive K values (k0 + i) of a complex column.  Positions past K
+// and columns past ncol repeat the last valid one: they leave a column's
+// largest value alone, and their digits meet zero table digits or columns that
+// are not stored.  Unconditional loads stay one batch in flight; guarded ones
+// were compiled into a chain (16 loads took 16 latencies).
+template <bool INV, int NV>
+__device__ __forceinline__ void loadn(const I8Args &a, const Unit &u, int col, int k0, double2 (&x)[NV])
+{
+  col = min(col, a.ncol - 1);
   if (!INV) {
-    const double2 *src = a.F + ((long long)u.m * a.ncol + (cv ? col : 0)) * a.J + u.p * a.JH;
+    const double2 *src = a.F + ((long long)u.m * a.ncol + col) * a.J + u.p * a.JH;
+    if (u.K % 2 == 0) {
 #pragma unroll
-    for (int i = 0; i < NV; ++i) x[i] = (cv && k0 + i < u.K) ? src[k0 + i] : make_double2(0.0, 0.0);
+      for (int i = 0; i < NV; i += 2) ldg32(src + min(k0 + i, u.K - 2), x[i], x[i + 1]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < NV; ++i) x[i] = src[min(k0 + i, u.K - 1)];
+    }
   } else {
     // one row pointer advanced by two internal rows (one parity) per value:
     // no per-value 64-bit index products held for the whole batch of loads
     const size_t step = (size_t)2 * a.ncol;
-    const double2 *src = a.Sc + ((long long)u.rowoff + u.p + 2 * k0) * a.ncol + (cv ? col : 0);
-    const int nv = cv ? u.K - k0 : 0;
+    const double2 *src = a.Sc + ((long long)u.rowoff + u.p + 2 * min(k0, u.K - 1)) * a.ncol + col;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-      x[i] = i < nv ? *src : make_double2(0.0, 0.0);
-      src += step;
+      x[i] = *src;
+      src += k0 + i + 1 < u.K ? step : 0;
     }
   }
 }
-template <bool INV>
-__device__ __forceinline__ void load16(const I8Args &a, const Unit &u, int col, bool cv, int k0, double2 (&x)[16])
-{
-  loadn<INV, 16>(a, u, col, cv, k0, x);
-}
-
 // r, im <- the largest high word (sign cleared) of the real and imaginary
 // parts of NV values and r, im
 template <int NV>
@@ -497,35 +599,51 @@ template <bool INV, bool CACHE>
 __device__ void role_convert(const I8Args &a, const Ctl &c, unsigned char *As, int *exps, const Lut &t, Unit u, bool have, int g1)
 {
   using R = Roles<INV>;
+  constexpr bool SCAN = scan_of(INV, CACHE);
   constexpr int kPass = 8 / R::kConvW;  // column passes: 64 columns, 8 per warp and pass
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c8 = lane & 7, q = lane >> 3;
   // half of the lanes write the imaginary row first, so that each 8-lane
   // phase of a 16-byte store covers the eight rows of a core matrix
   const int first_part = (c8 >> 2) & 1;
-  static_assert(kPass <= 2, "two exponent pairs per thread");
-  int er0 = 0, ei0 = 0, er1 = 0, ei1 = 0;  // column exponents of passes 0 and 1
-  int k = 0;
-  for (; have; have = next_unit<INV>(a, t, g1, u), ++k) {
-    const int st = k & 1;
-    if (CACHE && unit_cached(u)) {
-      // the producer copies these digits from the cache; the converters still
-      // step through the stage's phases one at a time (a parity wait only
-      // tells the last two phases apart), so they wait for unit k - 2 here
-      if (k >= 2 && !warp_wait(c, B_DEMPTY + st, ((k >> 1) - 1) & 1)) break;
-      continue;
-    }
-    const int k0 = u.ch * kKC + 16 * q;
-    // a sub-item with more than two segments keeps its digits for its later groups
-    uint8_t *const cache = (CACHE && u.nseg > 2) ? cache_stage(a, u) : nullptr;
+  const int cw = 8 * (warp - R::kConv0) + c8;
+  int er[kPass], ei[kPass];  // column exponents of the passes (selects: the pass loop is not unrolled)
+  auto pick = [](const int (&e)[kPass], int ps) {
+    int v = e[0];
+#pragma unroll
+    for (int i = 1; i < kPass; ++i) v = ps == i ? e[i] : v;
+    return v;
+  };
+  auto set = [](int (&e)[kPass], int ps, int v) {
+#pragma unroll
+    for (int i = 0; i < kPass; ++i) e[i] = ps == i ? v : e[i];
+  };
+  uint32_t epar = 0;  // parity of each stage's next release
+  for (; have; have = next_unit<INV, CACHE>(a, t, g1, u)) {
+    const int f = u.fill_base + u.fill, st = f & 1;
     const bool first = u.seg == 0 && u.ch == 0;
     const int slot = u.sub_count & (kSlots - 1);
-    if (first && u.sub_count >= kSlots && !warp_wait(c, B_EEMPTY + slot, (u.sub_count / kSlots - 1) & 1)) break;
-    bool ok = true, stage_free = k < 2;
+    if constexpr (SCAN) {
+      if (first) {
+        if (!warp_wait(c, B_EFULL + slot, (u.sub_count / kSlots) & 1)) break;
+#pragma unroll
+        for (int ps = 0; ps < kPass; ++ps) {
+          const int2 e = *reinterpret_cast<const int2 *>(exps + slot * kM + 2 * (cw + 8 * R::kConvW * ps));
+          er[ps] = e.x;
+          ei[ps] = e.y;
+        }
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(c.bar + B_EEMPTY + slot);
+      }
+    }
+    if (CACHE && u.seg > 0) continue;  // later groups: from the stages or the cache
+    const int k0 = u.chunk * kKC + 16 * q;
+    if (!SCAN && first && u.sub_count >= kSlots && !warp_wait(c, B_EEMPTY + slot, (u.sub_count / kSlots - 1) & 1)) break;
+    bool ok = true, stage_free = f < 2;
     unsigned char *stage = As + st * kStageA;
 #pragma unroll 1
     for (int ps = 0; ps < kPass; ++ps) {
-      const int cl = 8 * (warp - R::kConv0) + c8 + 8 * R::kConvW * ps;  // complex column within the tile
+      const int cl = cw + 8 * R::kConvW * ps;  // complex column within the tile
       const int col = u.col0 + cl;
       const bool cv = col < a.ncol;
       // the exponent of a column's largest magnitude is that of the largest
@@ -549,7 +667,7 @@ __device__ void role_convert(const I8Args &a, const Ctl &c, unsigned char *As, i
         r = max(r, hr[0]);
         im = max(im, hi[0]);
       };
-      if (first) {
+      if (!SCAN && first) {
         // column exponents over the sub-item's other K chunks (the first
         // unit converts chunk 0), kPreBatch values of this thread in flight
         // at a time, before this chunk's values take their registers
@@ -558,20 +676,21 @@ __device__ void role_convert(const I8Args &a, const Ctl &c, unsigned char *As, i
 #pragma unroll 1
           for (int i0 = 0; i0 < 16; i0 += PB) {
             double2 y[PB];
-            loadn<INV, PB>(a, u, col, cv, kc * kKC + 16 * q + i0, y);
+            loadn<INV, PB>(a, u, col, kc * kKC + 16 * q + i0, y);
             hmaxn<PB>(y, mr, mi);
           }
       }
       double2 x[16];
-      load16<INV>(a, u, col, cv, k0, x);
-      if (first) {
+      loadn<INV, 16>(a, u, col, k0, x);
+      if (!SCAN && first) {
         hmax(x, mr, mi);
         mr = max(mr, __shfl_xor_sync(0xffffffffu, mr, 8));
         mr = max(mr, __shfl_xor_sync(0xffffffffu, mr, 16));
         mi = max(mi, __shfl_xor_sync(0xffffffffu, mi, 8));
         mi = max(mi, __shfl_xor_sync(0xffffffffu, mi, 16));
         const int e_r = i8::exp_of_hi(mr), e_i = i8::exp_of_hi(mi);
-        if (ps) { er1 = e_r; ei1 = e_i; } else { er0 = e_r; ei0 = e_i; }
+        set(er, ps, e_r);
+        set(ei, ps, e_i);
         if (q == 0) {
           exps[slot * kM + 2 * cl] = e_r;
           exps[slot * kM + 2 * cl + 1] = e_i;
@@ -586,7 +705,8 @@ __device__ void role_convert(const I8Args &a, const Ctl &c, unsigned char *As, i
           if (k0 + 8 * h + 8 <= u.K) l2::discard_line(src + 8 * h);
       }
       if (!stage_free) {
-        if (!warp_wait(c, B_DEMPTY + st, ((k >> 1) - 1) & 1)) { ok = false; break; }
+        if (!warp_wait(c, B_DEMPTY + st, (epar >> st) & 1)) { ok = false; break; }
+        epar ^= 1u << st;
         stage_free = true;
       }
       // K positions at or past K meet zero table digits, so whatever the stage
@@ -595,7 +715,7 @@ __device__ void role_convert(const I8Args &a, const Ctl &c, unsigned char *As, i
 #pragma unroll
       for (int pp = 0; pp < 2; ++pp) {
         const int part = pp ^ first_part;
-        const double sc = i8::pow2(i8::kBitsData - (part ? (ps ? ei1 : ei0) : (ps ? er1 : er0)));
+        const double sc = i8::pow2(i8::kBitsData - (part ? pick(ei, ps) : pick(er, ps)));
         // four values at a time: conversions, then their byte permutes (the
         // groups are independent, and fewer words are live at once)
         uint32_t w[4][kDigitsData];
@@ -615,27 +735,65 @@ __device__ void role_convert(const I8Args &a, const Ctl &c, unsigned char *As, i
         for (int s = 0; s < kDigitsData; ++s) {
           const uint4 d4 = make_uint4(w[0][s], w[1][s], w[2][s], w[3][s]);
           *reinterpret_cast<uint4 *>(stage + s * kTileA + off) = d4;
-          if (cache) *reinterpret_cast<uint4 *>(cache + s * kTileA + off) = d4;
         }
       }
     }
     if (!ok) break;
-    if (first) {
+    if (!SCAN && first) {
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(c.bar + B_EFULL + slot);
     }
     tc::fence_proxy_async();
-    if (cache) tc::fence_proxy_async_global();
     __syncwarp();
-    if (lane == 0) {
-      tc::mbar_arrive(c.bar + B_DFULL + st);
-      // the sub-item's first group is written to the cache: its later groups may be copied
-      if (cache && u.ch == u.nch - 1) tc::mbar_arrive(c.bar + B_SREADY + (u.csub & 1));
-    }
+    if (lane == 0) tc::mbar_arrive(c.bar + B_DFULL + st);
   }
 }
 
-template <bool INV>
+// The column exponents of the synthesis with the digit cache: two warps read
+// each sub-item's data once, kAhead sub-items before the epilogue, and the
+// converters then find it in L2.  Warp h takes columns 32 h to 32 h + 31, lane l
+// keeps column 32 h + l.
+template <bool INV, bool CACHE>
+__device__ void role_scan(const I8Args &a, const Ctl &c, int *exps, const Lut &t, Unit u, bool have, int g1)
+{
+  const int lane = threadIdx.x & 31, h = (threadIdx.x >> 5) - Roles<INV>::kScan0;
+  while (have) {
+    const int n = u.sub_count, slot = n & (kSlots - 1);
+    // the readers have taken the exponents of sub-item n - kAhead; a slot is
+    // filled again only kSlots sub-items later, so this phase is never two back
+    if (n >= kAhead && !warp_wait(c, B_EEMPTY + ((n - kAhead) & (kSlots - 1)), ((n - kAhead) / kSlots) & 1)) break;
+    int mr = 0, mi = 0;
+    const int col = u.col0 + 32 * h;
+    // strided rows, contiguous over the columns; only the high words are
+    // loaded, half the registers per value in flight
+    const double2 *src = a.Sc + ((long long)u.rowoff + u.p) * a.ncol + min(col + lane, a.ncol - 1);
+    const size_t step = (size_t)2 * a.ncol;
+#pragma unroll 1
+    for (int k0 = 0; k0 < u.K; k0 += 32) {
+      int x[32], y[32];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        x[i] = __ldg(reinterpret_cast<const int *>(src) + 1) & 0x7FFFFFFF;
+        y[i] = __ldg(reinterpret_cast<const int *>(src) + 3) & 0x7FFFFFFF;
+        src += k0 + i + 1 < u.K ? step : 0;
+      }
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        mr = max(mr, x[i]);
+        mi = max(mi, y[i]);
+      }
+    }
+    exps[slot * kM + 2 * (32 * h + lane)] = i8::exp_of_hi(mr);
+    exps[slot * kM + 2 * (32 * h + lane) + 1] = i8::exp_of_hi(mi);
+    __syncwarp();
+    if (lane == 0) tc::mbar_arrive(c.bar + B_EFULL + slot);
+    u.ch = u.nch - 1;  // on to the next sub-item (its fill_base is not used here)
+    u.seg = u.nseg;
+    have = next_unit<INV, CACHE>(a, t, g1, u);
+  }
+}
+
+template <bool INV, bool CACHE>
 __device__ void role_epilogue(const I8Args &a, const Ctl &c, const int *exps, uint32_t tbase, const Lut &t, Unit u, bool have, int g1)
 {
   using R = Roles<INV>;
@@ -647,7 +805,7 @@ __device__ void role_epilogue(const I8Args &a, const Ctl &c, const int *exps, ui
   const uint32_t tl = tbase + ((uint32_t)(32 * quad) << 16);
   const uint64_t keep = l2::keep_policy();
   int ecol = 0;
-  for (; have; have = next_unit<INV>(a, t, g1, u)) {
+  for (; have; have = next_unit<INV, CACHE>(a, t, g1, u)) {
     const int col = u.col0 + cl;
     const bool cv = col < a.ncol;
     if (u.seg == 0 && u.ch == 0) {
@@ -661,7 +819,6 @@ __device__ void role_epilogue(const I8Args &a, const Ctl &c, const int *exps, ui
     const int s0 = u.seg, s1 = min(u.seg + 2, u.nseg);
     const double *frow = a.tfac + u.teoff;
     const double fcol = i8::pow2(ecol < 1023 ? ecol : 1023);
-    const bool fast = u.K <= 64;
     bool ok = true;
     for (int s = s0; s < s1; ++s) {
       const int npad = seg_npad(u.nrow, s);
@@ -680,7 +837,7 @@ __device__ void role_epilogue(const I8Args &a, const Ctl &c, const int *exps, ui
 #pragma unroll
         for (int L = 0; L < kLevels; ++L) tc::tmem_ld4(tl + (uint32_t)(set * kSetCols + L * npad + 4 * g4), r[L]);
         tc::tmem_wait_ld();
-        if (fast)
+        if (!CACHE && u.K <= i8::kPairK)
           epilogue_rows<INV, true>(a, u, s * kSeg + 4 * g4, col, cv, part, r, fr, fcol, keep);
         else
           epilogue_rows<INV, false>(a, u, s * kSeg + 4 * g4, col, cv, part, r, fr, fcol, keep);
@@ -694,7 +851,7 @@ __device__ void role_epilogue(const I8Args &a, const Ctl &c, const int *exps, ui
 }
 
 template <bool INV, bool CACHE>
-__global__ void __launch_bounds__(kThreads, 1) k_leg_i8(I8Args a)
+__global__ void __launch_bounds__(threads_of(scan_of(INV, CACHE)), 1) k_leg_i8(I8Args a)
 {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ __align__(8) uint64_t bar[B_COUNT];
@@ -734,13 +891,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_leg_i8(I8Args a)
       tc::mbar_init(bar + B_AEMPTY + i, Roles<INV>::kEpiW);
     }
     for (int i = 0; i < kSlots; ++i) {
-      tc::mbar_init(bar + B_EFULL + i, Roles<INV>::kConvW);
-      tc::mbar_init(bar + B_EEMPTY + i, Roles<INV>::kEpiW);
+      tc::mbar_init(bar + B_EFULL + i, scan_of(INV, CACHE) ? kScanW : Roles<INV>::kConvW);
+      tc::mbar_init(bar + B_EEMPTY + i, Roles<INV>::kEpiW + (scan_of(INV, CACHE) ? Roles<INV>::kConvW : 0));
     }
     for (int i = 0; i < 2; ++i) {
       tc::mbar_init(bar + B_CFULL + i, 1);
-      tc::mbar_init(bar + B_SREADY + i, Roles<INV>::kConvW);
+      tc::mbar_init(bar + B_CEMPTY + i, 1);
     }
+    tc::mbar_init(bar + B_SREADY, 1);
     tc::mbar_init(bar + B_DONE, 1);
     abort_flag = 0;
     tc::mbar_fence_init();
@@ -759,8 +917,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_leg_i8(I8Args a)
     if (lane == 0) role_mma<INV, CACHE>(a, c, tc::smem_addr(As), tc::smem_addr(Ps), tbase, t, u, have, g1);
   } else if (warp < Roles<INV>::kEpi0) {
     role_convert<INV, CACHE>(a, c, As, exps, t, u, have, g1);
-  } else {
-    role_epilogue<INV>(a, c, exps, tbase, t, u, have, g1);
+  } else if (warp < Roles<INV>::kScan0) {
+    role_epilogue<INV, CACHE>(a, c, exps, tbase, t, u, have, g1);
+  } else if constexpr (scan_of(INV, CACHE)) {
+    role_scan<INV, CACHE>(a, c, exps, t, u, have, g1);
   }
 
   tc::fence_before();
@@ -826,7 +986,7 @@ int build_i8_tables(sht_plan *p)
   for (int d = 0; d < 2; ++d) {
     const int nrow = d ? JH : (N + 3) / 2, K = d ? (N + 3) / 2 : JH;
     if (nrow <= 2 * kSeg) continue;
-    t->scr_cta[d] = 2LL * ((K + kKC - 1) / kKC) * kStageA;
+    t->scr_cta[d] = (long long)((K + kKC - 1) / kKC) * kStageA;
     const size_t bytes = (size_t)t->scr_cta[d] * (p->num_sms > 0 ? p->num_sms : 1);
     if ((e = cudaMalloc(&t->scr[d], bytes)) != cudaSuccess) return fail(e, "split digit cache");
   }
@@ -878,9 +1038,10 @@ int launch_i8(sht_plan *p, bool inverse, const double2 *in, int ncol, double2 *o
     set_error("split precision: the truncation's lookup tables do not fit beside the stages");
     return SHT_ERR_UNSUPPORTED_SIZE;
   }
-  cudaError_t e = kernel_setup((const void *)kern, smem, kThreads);
+  const int threads = threads_of(scan_of(inverse, a.scr != nullptr));
+  cudaError_t e = kernel_setup((const void *)kern, smem, threads);
   if (e != cudaSuccess) return cuda_fail(e, "split smem attribute");
-  kern<<<grid, kThreads, smem, s>>>(a);
+  kern<<<grid, threads, smem, s>>>(a);
   count_launch();
   e = cudaGetLastError();
   return e == cudaSuccess ? SHT_OK : cuda_fail(e, inverse ? "k_leg_i8<inv>" : "k_leg_i8<fwd>");

@@ -183,6 +183,17 @@ __device__ __forceinline__ void bulk_g2s(void *dst_smem, const void *src, uint32
                : "memory");
 }
 
+// Bulk copy shared -> global of `bytes` (the same rules), in the issuing
+// thread's bulk group; wait_read: the sources may be overwritten; wait: the
+// writes are done.
+__device__ __forceinline__ void bulk_s2g(void *dst, uint32_t src_smem, uint32_t bytes)
+{
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n" ::"l"(dst), "r"(src_smem), "r"(bytes) : "memory");
+  asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+}
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait() { asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory"); }
+
 __device__ __forceinline__ uint64_t globaltimer_ns()
 {
   uint64_t t;
