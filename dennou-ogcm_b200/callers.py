@@ -16,6 +16,19 @@ have, for comparison and timing.
 """
 from __future__ import annotations
 
+from .spmlutil import SpmlUtil
+
+
+def _spectra(sp, *ws):
+    """Whether ws are results of this package's plan that the fused tails may
+    overwrite: plain CUDA float64 (K, lm) tensors."""
+    if not isinstance(sp, SpmlUtil):
+        return False
+    import torch
+
+    return all(type(w) is torch.Tensor and w.is_cuda and w.dim() == 2 and w.dtype == torch.float64 and w.is_contiguous()
+               and w.shape == ws[0].shape for w in ws)
+
 
 def htrc_rhs(sp, u, v, tmp, vflx_div, adv_filter, h_phys):
     """Tracer tendency of HBEBaroc_HTRCRHS (HBEBaroc_hspm_vfvm_mod.f90:160-172):
@@ -27,9 +40,28 @@ def htrc_rhs(sp, u, v, tmp, vflx_div, adv_filter, h_phys):
     given per level.  Three transform calls for all levels: the flux
     divergence with its products formed in the longitude transform, the
     analysis of the vertical term and the synthesis."""
-    w = sp.w_xy(vflx_div) - sp.w_AlphaOptrProd_xy(u, v, tmp)
-    w *= adv_filter[None, :]
+    w, adv = sp.w_xy(vflx_div), sp.w_AlphaOptrProd_xy(u, v, tmp)
+    if _spectra(sp, w, adv) and _row(adv_filter, w):
+        sp._sub_filter(w, adv, adv_filter)
+    else:
+        w = w - adv
+        w *= adv_filter[None, :]
     return sp.xy_w(w) + h_phys
+
+
+def _row(f, w):
+    """Whether f is a plain vector of w's row length on w's device."""
+    return (type(f) is type(w) and f.is_cuda and f.device == w.device and f.dtype == w.dtype and f.dim() == 1
+            and f.shape[0] == w.shape[1] and f.is_contiguous() and not f.requires_grad)
+
+
+def _tendencies(sp, wv, wd, c):
+    """calc_VorDiv2UV(-wd, wv - w_Lapla_w(w_xy(c))), wv and wd overwritten where the one-pass tail applies."""
+    wc = sp.w_xy(c)
+    if _spectra(sp, wv, wd, wc):
+        sp._sub_lapla(wv, wd, wc)
+        return sp.calc_VorDiv2UV(wd, wv)
+    return sp.calc_VorDiv2UV(-wd, wv - sp.w_Lapla_w(wc))
 
 
 def momrhs_vordiv(sp, a, b, c):
@@ -44,8 +76,7 @@ def momrhs_vordiv(sp, a, b, c):
     calc_UVCosLat2VorDiv(A, B) returns (H(B, -A), H(A, B)) with H =
     w_AlphaOptr_xy, i.e. (w_Div_RHS + Lapla term, -w_Vor_RHS) from one
     analysis of both fields.  Four calls for all levels."""
-    vor, div = sp.calc_UVCosLat2VorDiv(a, b)
-    return sp.calc_VorDiv2UV(-div, vor - sp.w_Lapla_w(sp.w_xy(c)))
+    return _tendencies(sp, *sp.calc_UVCosLat2VorDiv(a, b), c)
 
 
 def momrhs_vordiv_fma(sp, u, v, vor, za, zb, c):
@@ -57,8 +88,7 @@ def momrhs_vordiv_fma(sp, u, v, vor, za, zb, c):
     products, e.g. CoriU + VAdvV/H - VRHS_phys + DensEdd GradLat(GeoPot)/(rho a)),
     with the products formed while the grids load into the longitude
     transform, so that A and B are never written."""
-    wv, wd = sp.calc_UVCosLat2VorDiv_fma(u, v, vor, za, zb)
-    return sp.calc_VorDiv2UV(-wd, wv - sp.w_Lapla_w(sp.w_xy(c)))
+    return _tendencies(sp, *sp.calc_UVCosLat2VorDiv_fma(u, v, vor, za, zb), c)
 
 
 def diagnose_vordiv(sp, u, v):

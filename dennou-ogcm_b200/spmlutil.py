@@ -114,6 +114,8 @@ def load_library(path: str | None = None):
         getattr(lib, "sht_synthesis" + suf).argtypes = [_VP, _VP, ctypes.c_int, ctypes.c_int, _VP, ctypes.c_int,
                                                         ctypes.c_int, ctypes.c_int]
     lib.sht_wa_diffuse_to_dev.argtypes = [_VP, _VP, ctypes.c_int, _VP, ctypes.c_double, _VP, _VP]
+    lib.sht_wa_sub_filter_dev.argtypes = [_VP, _VP, _VP, ctypes.c_int, _VP]
+    lib.sht_wa_sub_lapla_dev.argtypes = [_VP, _VP, _VP, _VP, ctypes.c_int]
     lib.sht_roundtrip_diffuse_dev.argtypes = [_VP, _VP, ctypes.c_int, _VP, ctypes.c_double, _VP]
     lib.sht_plan_l_nm.argtypes = [_VP, ctypes.c_int, ctypes.c_int]
     lib.sht_plan_nm_l.argtypes = [_VP, ctypes.c_int, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int)]
@@ -459,6 +461,22 @@ class SpmlUtil:
                                     _VP(f.ctypes.data) if f is not None else None)
         _check(st, "diffuse")
         return out
+
+    def _sub_filter(self, wa, wb, filt):
+        """wa <- filt (wa - wb) in place (CUDA float64, contiguous, (nb, lm))."""
+        self._set_torch_stream(wa)
+        st = _lib.sht_wa_sub_filter_dev(self._h, wa.data_ptr(), wb.data_ptr(), wa.shape[0], filt.data_ptr())
+        if st != SHT_OK:
+            _check(st, "sub_filter")
+        return wa
+
+    def _sub_lapla(self, wa, wneg, wc):
+        """wa <- wa - Lapla(wc), wneg <- -wneg in place (CUDA float64, contiguous, (nb, lm))."""
+        self._set_torch_stream(wa)
+        st = _lib.sht_wa_sub_lapla_dev(self._h, wa.data_ptr(), wneg.data_ptr(), wc.data_ptr(), wa.shape[0])
+        if st != SHT_OK:
+            _check(st, "sub_lapla")
+        return wa, wneg
 
     # ------------------------------------ haloed arrays (leading dimensions)
     def _section(self, x, i0, j0, name):

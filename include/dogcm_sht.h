@@ -305,6 +305,11 @@ SHT_API int sht_wa_diffuse_dev(sht_plan *plan, double *wa, int nb, const double 
 /* the same into another array (out may be wa) */
 SHT_API int sht_wa_diffuse_to_dev(sht_plan *plan, const double *wa, int nb, const double *coef, double dt,
                           const double *filter, double *out);
+/* the spectral tails of the tracer and momentum tendencies, in place on
+ * distinct arrays:  wa <- filter (wa - wb)  (filter: lm entries), and
+ * wa <- wa - Lapla(wc), wneg <- -wneg */
+SHT_API int sht_wa_sub_filter_dev(sht_plan *plan, double *wa, const double *wb, int nb, const double *filter);
+SHT_API int sht_wa_sub_lapla_dev(sht_plan *plan, double *wa, double *wneg, const double *wc, int nb);
 SHT_API int sht_avrlonlat_xya_dev(sht_plan *plan, const double *xya, int nb, double *out);
 SHT_API int sht_intlonlat_xya_dev(sht_plan *plan, const double *xya, int nb, double *out);
 SHT_API int sht_ya_avrlon_xya_dev(sht_plan *plan, const double *xya, int nb, double *out);
