@@ -161,21 +161,29 @@ __global__ void __launch_bounds__(RowShape<R1, H, JTh>::NT, MINB) k_row_fwd(FftA
     const double2 *src = reinterpret_cast<const double2 *>(gb) + off;
 #pragma unroll
     for (int n = LO; n < HI; ++n) v[n] = valid ? __ldcs(src + R2 * n) : make_double2(0.0, 0.0);
-    if (MUL) {
-      const double2 *fr = reinterpret_cast<const double2 *>(a.mul + (long long)(col % a.nmul) * IJ) + off;
+  };
+  // the factors when the tile's turn comes, so that its prefetched rows are not
+  // waited for before the unpack (products of two fields, T85 pairs, 480:
+  // 103 -> 99 us; T341 rows, 48: 214 -> 191; no size slower)
+  auto multiply = [&](unsigned t) {
+    int col, h0;
+    where(t, col, h0);
+    const int jh = h0 + r % JTh, j = r < JTh ? a.JH + jh : a.JH - 1 - jh;
+    const bool valid = jh < a.JH;
+    const long long off = (long long)(valid ? j : 0) * NC + u;
+    const double2 *fr = reinterpret_cast<const double2 *>(a.mul + (long long)(col % a.nmul) * IJ) + off;
 #pragma unroll
-      for (int n = LO; n < HI; ++n) {
-        const double2 q = valid ? __ldg(fr + R2 * n) : make_double2(0.0, 0.0);
-        v[n] = make_double2(v[n].x * q.x, v[n].y * q.y);
-      }
-      if (a.add0) {
-        const double *zb = col < a.nsplit ? a.add0 + (long long)col * IJ : a.add1 + (long long)(col - a.nsplit) * IJ;
-        const double2 *zr = reinterpret_cast<const double2 *>(zb) + off;
+    for (int n = 0; n < R1; ++n) {
+      const double2 q = valid ? __ldg(fr + R2 * n) : make_double2(0.0, 0.0);
+      v[n] = make_double2(v[n].x * q.x, v[n].y * q.y);
+    }
+    if (a.add0) {
+      const double *zb = col < a.nsplit ? a.add0 + (long long)col * IJ : a.add1 + (long long)(col - a.nsplit) * IJ;
+      const double2 *zr = reinterpret_cast<const double2 *>(zb) + off;
 #pragma unroll
-        for (int n = LO; n < HI; ++n) {
-          const double2 z = valid ? __ldg(zr + R2 * n) : make_double2(0.0, 0.0);
-          v[n] = make_double2(v[n].x + z.x, v[n].y + z.y);
-        }
+      for (int n = 0; n < R1; ++n) {
+        const double2 z = valid ? __ldg(zr + R2 * n) : make_double2(0.0, 0.0);
+        v[n] = make_double2(v[n].x + z.x, v[n].y + z.y);
       }
     }
   };
@@ -190,6 +198,7 @@ __global__ void __launch_bounds__(RowShape<R1, H, JTh>::NT, MINB) k_row_fwd(FftA
     int col, h0;
     where(t, col, h0);
     if constexpr (PF < R1) load(t, pf, all);
+    if (MUL) multiply(t);
     pass_a_store<R1, T, false>(v, buf + r * RS + u, S, stw, u);
     __syncthreads();
     {
@@ -390,25 +399,31 @@ __global__ void __launch_bounds__(PairShape<R1, H, JTh>::NT, MINB) k_pair_fwd(Ff
 #pragma unroll
     for (int n = 0; n < R1; ++n)
       v[n] = valid ? make_double2(__ldcs(gb + on + R2 * n), __ldcs(gb + os + R2 * n)) : make_double2(0.0, 0.0);
-    if (MUL) {
-      const double *f = a.mul + (long long)(col % a.nmul) * IJ;
+  };
+  // the factors when the tile's turn comes (see k_row_fwd)
+  auto multiply = [&](unsigned t) {
+    int col, h0;
+    where(t, col, h0);
+    const bool valid = h0 + r < a.JH;
+    const int jn = a.JH + (valid ? h0 + r : 0), js = 2 * a.JH - 1 - jn;
+    const int on = jn * I + u, os = js * I + u;
+    const double *f = a.mul + (long long)(col % a.nmul) * IJ;
+#pragma unroll
+    for (int n = 0; n < R1; ++n) {
+      v[n].x *= __ldg(f + on + R2 * n);
+      v[n].y *= __ldg(f + os + R2 * n);
+    }
+    if (a.add0) {
+      const double *z = col < a.nsplit ? a.add0 + (long long)col * IJ : a.add1 + (long long)(col - a.nsplit) * IJ;
 #pragma unroll
       for (int n = 0; n < R1; ++n) {
-        v[n].x *= __ldg(f + on + R2 * n);
-        v[n].y *= __ldg(f + os + R2 * n);
+        v[n].x += __ldg(z + on + R2 * n);
+        v[n].y += __ldg(z + os + R2 * n);
       }
-      if (a.add0) {
-        const double *z = col < a.nsplit ? a.add0 + (long long)col * IJ : a.add1 + (long long)(col - a.nsplit) * IJ;
-#pragma unroll
-        for (int n = 0; n < R1; ++n) {
-          v[n].x += __ldg(z + on + R2 * n);
-          v[n].y += __ldg(z + os + R2 * n);
-        }
-      }
-      if (!valid)
-#pragma unroll
-        for (int n = 0; n < R1; ++n) v[n] = make_double2(0.0, 0.0);
     }
+    if (!valid)
+#pragma unroll
+      for (int n = 0; n < R1; ++n) v[n] = make_double2(0.0, 0.0);
   };
   const uint64_t keep = l2::keep_policy();
   unsigned t = blockIdx.x;
@@ -417,6 +432,7 @@ __global__ void __launch_bounds__(PairShape<R1, H, JTh>::NT, MINB) k_pair_fwd(Ff
   for (; t < ntot; t += gridDim.x) {
     int col, h0;
     where(t, col, h0);
+    if (MUL) multiply(t);
     pass_a_store<R1, T, false>(v, buf + r * RS + u, S, stw, u);
     __syncthreads();
     {
