@@ -31,6 +31,8 @@
 // are chosen below for the phases whose lanes run over the rows.
 #include "sht_fft_row.cuh"
 
+#include <type_traits>
+
 namespace sht {
 
 namespace {
@@ -126,7 +128,7 @@ __device__ __forceinline__ void pass_a_store(double2 (&v)[R1], double2 *o, int S
   }
 }
 
-template <int R1, int H, int JTh, int MUL, int MINB>
+template <int R1, int H, int JTh, int MUL, int MINB, int PF>
 __global__ void __launch_bounds__(RowShape<R1, H, JTh>::NT, MINB) k_row_fwd(FftArgs a)
 {
   using P = RowShape<R1, H, JTh>;
@@ -147,7 +149,8 @@ __global__ void __launch_bounds__(RowShape<R1, H, JTh>::NT, MINB) k_row_fwd(FftA
     col = a.mul_pair ? (int)(c2 >> 1) + (int)(c2 & 1) * a.nsplit : (int)c2;
   };
   double2 v[R1];
-  auto load = [&](unsigned t) {
+  auto load = [&](unsigned t, auto lo, auto hi) {
+    constexpr int LO = decltype(lo)::value, HI = decltype(hi)::value;
     int col, h0;
     where(t, col, h0);
     const int jh = h0 + r % JTh, j = r < JTh ? a.JH + jh : a.JH - 1 - jh;
@@ -157,11 +160,11 @@ __global__ void __launch_bounds__(RowShape<R1, H, JTh>::NT, MINB) k_row_fwd(FftA
     const long long off = (long long)(valid ? j : 0) * NC + u;
     const double2 *src = reinterpret_cast<const double2 *>(gb) + off;
 #pragma unroll
-    for (int n = 0; n < R1; ++n) v[n] = valid ? __ldcs(src + R2 * n) : make_double2(0.0, 0.0);
+    for (int n = LO; n < HI; ++n) v[n] = valid ? __ldcs(src + R2 * n) : make_double2(0.0, 0.0);
   };
   // the factors when the tile's turn comes, so that its prefetched rows are not
   // waited for before the unpack (products of two fields, T85 pairs, 480:
-  // 103 -> 99 us; T341 rows, 48: 214 -> 185; no size slower)
+  // 103 -> 99 us; T341 rows, 48: 214 -> 191; no size slower)
   auto multiply = [&](unsigned t) {
     int col, h0;
     where(t, col, h0);
@@ -186,11 +189,15 @@ __global__ void __launch_bounds__(RowShape<R1, H, JTh>::NT, MINB) k_row_fwd(FftA
   };
   const uint64_t keep = l2::keep_policy();
   unsigned t = blockIdx.x;
-  if (t < ntot) load(t);
+  constexpr std::integral_constant<int, 0> zero{};
+  constexpr std::integral_constant<int, PF> pf{};
+  constexpr std::integral_constant<int, R1> all{};
+  if (t < ntot) load(t, zero, pf);
   __syncthreads();  // the twiddle tables are in
   for (; t < ntot; t += gridDim.x) {
     int col, h0;
     where(t, col, h0);
+    if constexpr (PF < R1) load(t, pf, all);
     if (MUL) multiply(t);
     pass_a_store<R1, T, false>(v, buf + r * RS + u, S, stw, u);
     __syncthreads();
@@ -201,7 +208,7 @@ __global__ void __launch_bounds__(RowShape<R1, H, JTh>::NT, MINB) k_row_fwd(FftA
 #pragma unroll
       for (int k = 0; k < R1; ++k) own[H * k] = z[k];
     }
-    if (t + gridDim.x < ntot) load(t + gridDim.x);
+    if (t + gridDim.x < ntot) load(t + gridDim.x, zero, pf);
     __syncthreads();
     // X_m = E - i W^m D, E/D = (Z_m +- conj Z_{NC-m})/2, of the pair's two rows
     const int i = tid % JTh;
@@ -565,11 +572,11 @@ int launch_rows(void (*kern)(FftArgs), int threads, size_t smem, int pairs, cons
   return e == cudaSuccess ? SHT_OK : cuda_fail(e, name);
 }
 
-template <int R1, int H, int JTh, int MINB>
+template <int R1, int H, int JTh, int MINB, int PF>
 int row_fwd(const sht_plan *p, const FftArgs &a, cudaStream_t s)
 {
   using P = RowShape<R1, H, JTh>;
-  return launch_rows(a.mul ? k_row_fwd<R1, H, JTh, 1, MINB> : k_row_fwd<R1, H, JTh, 0, MINB>, P::NT,
+  return launch_rows(a.mul ? k_row_fwd<R1, H, JTh, 1, MINB, PF> : k_row_fwd<R1, H, JTh, 0, MINB, PF>, P::NT,
                      P::smem(false, p->N), JTh, p, a, s, "k_row_fwd");
 }
 template <int R1, int H, int JTh, int MINB>
@@ -602,16 +609,16 @@ bool fft_row_supported(int NC, bool inverse) { return (NC >= 32 && NC <= 256) ||
 //   im = 128  rows, 3095                 70 / 73 -> 62 / 64
 //   im = 256  pairs, 480                 47 / 52 -> 43 / 45
 //   im = 512  rows, 720                  258 / 275 -> 258 / 237
-//   im = 1024 rows, 240                  510 -> 383 (two row pairs per block, three
-//             blocks per SM; four pairs, two blocks: 397; inverse with two pairs 422)
+//   im = 1024 rows, 240                  510 -> 397 (half of the next tile's
+//             rows prefetched; all of them spill: 432)
 int run_fft_row(bool inverse, const sht_plan *p, const FftArgs &a, cudaStream_t s)
 {
   switch (p->NC) {
   case 32: return pairs<8, 1, 16, 5, 6>(inverse, p, a, s);
-  case 64: return inverse ? row_inv<8, 1, 8, 6>(p, a, s) : row_fwd<8, 1, 8, 6>(p, a, s);
+  case 64: return inverse ? row_inv<8, 1, 8, 6>(p, a, s) : row_fwd<8, 1, 8, 6, 8>(p, a, s);
   case 128: return pairs<16, 1, 8, 3, 3>(inverse, p, a, s);
-  case 256: return inverse ? row_inv<16, 1, 4, 3>(p, a, s) : row_fwd<16, 1, 4, 3>(p, a, s);
-  case 512: if (!inverse) return row_fwd<16, 2, 2, 3>(p, a, s);  // fall through
+  case 256: return inverse ? row_inv<16, 1, 4, 3>(p, a, s) : row_fwd<16, 1, 4, 3, 16>(p, a, s);
+  case 512: if (!inverse) return row_fwd<16, 2, 4, 2, 8>(p, a, s);  // fall through
   default: set_error("fft: unsupported longitude count"); return SHT_ERR_UNSUPPORTED_SIZE;
   }
 }
