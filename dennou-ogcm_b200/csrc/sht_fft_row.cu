@@ -610,7 +610,9 @@ bool fft_row_supported(int NC, bool inverse) { return (NC >= 32 && NC <= 256) ||
 //   im = 256  pairs, 480                 47 / 52 -> 43 / 45
 //   im = 512  rows, 720                  258 / 275 -> 258 / 237
 //   im = 1024 rows, 240                  510 -> 397 (half of the next tile's
-//             rows prefetched; all of them spill: 432)
+//             rows prefetched; all of them spill: 432.  Two row pairs per block,
+//             three blocks: 384, but its 32-byte pieces per order lose where
+//             orders lie megabytes apart, 960: 1566 -> 1989)
 int run_fft_row(bool inverse, const sht_plan *p, const FftArgs &a, cudaStream_t s)
 {
   switch (p->NC) {

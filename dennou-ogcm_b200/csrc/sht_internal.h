@@ -213,10 +213,11 @@ int launch_leg_inv_fp64(const sht_plan *p, const double2 *S, int ncol, double2 *
 bool split_supported(const sht_plan *p);
 // Whether a contraction runs in split precision: always under SHT_PREC_SPLIT;
 // under SHT_PREC_AUTO when it is at least 128 terms long (jm/2 latitudes in
-// the analysis, (nm+3)/2 degrees of one parity in the synthesis), where the
-// int8 digit kernel measured faster than the FP64 tensor path on B200 (T170
-// analysis 0.41 against 0.44 ms; T341 3.09 / 2.77 against 3.78 / 3.52 ms; T170
-// synthesis, 86 terms, 0.48 against 0.40 ms).
+// the analysis, (nm+3)/2 degrees of one parity in the synthesis).  That is the
+// mode's documented meaning.  The line was drawn where the int8 digit kernel beat
+// the per-grid FP64 kernels of the time; the band kernels are now the faster on
+// both sides of it (T170, 720: 198 / 209 us against 412 / 324; T341, 960: 1758 /
+// 1792 against 2459 / 2403), so SHT_PREC_FP64 is the mode for speed.
 // --- whole plain transforms of small grids in one kernel (sht_small.cu)
 bool small_supported(const sht_plan *p);
 int launch_small_fwd(const sht_plan *p, const double *g, const double *const *gcol, int ncol, double *w,
@@ -234,8 +235,8 @@ inline bool use_split(const sht_plan *p, bool analysis)
 // plain analysis / synthesis by the single-kernel small-grid transform:
 // chosen with SHT_OPT_LEGENDRE_KERNEL = 4, and by the automatic choice for
 // im = 32 (16 complex points per row), the only size where it measured
-// faster than the batched kernels (T10, 480 field-levels: round trip 31
-// against 59 us); in FP64 only (split precision keeps the batched path)
+// faster than the batched kernels (T10, 480 field-levels: round trip 26
+// against 37 us); in FP64 only (split precision keeps the batched path)
 inline bool use_small(const sht_plan *p, bool analysis)
 {
   const bool want = p->leg_kernel == 4 || (p->leg_kernel == 0 && p->NC == 16);

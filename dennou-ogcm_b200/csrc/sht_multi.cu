@@ -8,10 +8,9 @@
 // forked from and joined into the batch's stream.  Each step kind is captured
 // once as a CUDA graph (fork, per-plan stages, join) and replayed.
 //
-// The tuner times, per plan, every Legendre variant that covers the grid
-// (paired persistent, latitude-chunked persistent and per-band FP64, and split
-// precision on the tensor cores when allowed) on the plan's own columns and
-// keeps the fastest.
+// The tuner times, per plan, the batched FP64 kernels, the single-kernel
+// transform of small grids and, when allowed, split precision on the plan's own
+// columns and keeps the fastest.
 //
 // Workspaces belong to the batch, not to the plans, so single-plan calls made
 // between runs cannot move memory that a captured graph refers to.

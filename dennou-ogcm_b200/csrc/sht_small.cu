@@ -23,10 +23,10 @@
 // (synthesis) with the same row factors, parities and SPML scaling (sqrt 2
 // for m > 0, SpmlUtil's wa layout) as the batched path.
 //
-// It is faster than the batched path only for the smallest grids (T10: 480
-// field-levels round trip 31 against 59 us): each block re-reads the Legendre
+// It is faster than the batched path only for the smallest grids (480
+// field-levels, round trip: T10 26 against 37 us, T21 45 against 28): each block re-reads the Legendre
 // table for its two levels, where the batched kernels use every table row on
-// 8 to 16 columns, and its phases (loads, transform, contraction, stores) run
+// 32 columns, and its phases (loads, transform, contraction, stores) run
 // one after the other in blocks that the shared-memory arrays keep few per SM.
 // The multi-instance tuner times it beside the batched kernels per plan.
 #include "sht_fft_tile.cuh"

@@ -282,7 +282,7 @@ contains
   !> Precision of the following transforms: SHT_PREC_FP64 (the default),
   !> SHT_PREC_SPLIT (integer digit products on the tensor cores, <= 1e-11
   !> relative) or SHT_PREC_AUTO (split where a contraction has at least 128
-  !> terms: the faster of the two per direction).  No counterpart in SPMODEL.
+  !> terms, FP64 below).  No counterpart in SPMODEL.
   subroutine b200_SetPrecision(mode)
     integer, intent(in) :: mode
     call check(sht_set_precision(plan, int(mode, c_int)), 'SetPrecision')

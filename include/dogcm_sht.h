@@ -62,11 +62,11 @@ extern "C" {
                              grid or spectral value, seven per table value),
                              exact integer digit products on the tcgen05
                              tensor cores, FP64 recombination                  */
-#define SHT_PREC_AUTO  2  /* per direction, the faster of the two on B200 as
-                             measured: split precision for a contraction of at
-                             least 128 terms (analysis: jm/2 latitudes;
+#define SHT_PREC_AUTO  2  /* per direction: split precision for a contraction
+                             of at least 128 terms (analysis: jm/2 latitudes;
                              synthesis: (nm+3)/2 degrees of one parity), FP64
-                             below.  Both meet the same 1e-11 bound.            */
+                             below.  Both meet the same 1e-11 bound.  The FP64
+                             kernels are the faster on both sides of the line.  */
 
 typedef struct sht_plan_s sht_plan;
 
