@@ -1030,8 +1030,29 @@ int sht_selftest_device_timeout(sht_plan *p, int limit_ms)
   std::lock_guard<std::mutex> lk(p->mtx);
   DeviceGuard g(p->device);
   if (!g.ok) { set_error("cudaSetDevice failed"); return SHT_ERR_CUDA; }
-  if ((rc = wait_selftest(p, (unsigned long long)limit_ms * 1000000ull))) return rc;
-  return device_error_status(p);
+  // one kernel's wait and word at a time: both have to raise their own
+  auto run = [&](auto launch, auto status, const char *what) {
+    int r = launch(p, (unsigned long long)limit_ms * 1000000ull, p->stream);
+    if (r) return r;
+    const cudaError_t e = cudaStreamSynchronize(p->stream);
+    if (e != cudaSuccess) return cuda_fail(e, what);
+    if ((r = status(p)) == SHT_OK) { set_error(std::string(what) + " recorded no timeout"); return (int)SHT_ERR_CUDA; }
+    return r;
+  };
+  rc = run(launch_split_wait_selftest, split_error_status, "device timeout self-test: the split kernel's wait");
+  if (rc != SHT_ERR_DEVICE_TIMEOUT) return rc;
+  return run(launch_band_wait_selftest, band_error_status, "device timeout self-test: the FP64 kernels' wait");
+}
+
+int sht_selftest_device_timeout_dev(sht_plan *p, int limit_ms)
+{
+  int rc = check_plan(p);
+  if (rc) return rc;
+  if (limit_ms < 1 || limit_ms > 1000) { set_error("limit_ms must be in 1..1000"); return SHT_ERR_INVALID_ARG; }
+  std::lock_guard<std::mutex> lk(p->mtx);
+  DeviceGuard g(p->device);
+  if (!g.ok) { set_error("cudaSetDevice failed"); return SHT_ERR_CUDA; }
+  return launch_band_wait_selftest(p, (unsigned long long)limit_ms * 1000000ull, p->stream);
 }
 
 int sht_set_stream(sht_plan *p, void *stream)

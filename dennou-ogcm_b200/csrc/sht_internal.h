@@ -255,8 +255,9 @@ int launch_leg_fwd_split(sht_plan *p, const double2 *F, int ncol, double2 *S, cu
 int launch_leg_inv_split(sht_plan *p, const double2 *S, int ncol, double2 *F, cudaStream_t s);
 void free_split_tables(sht_plan *p);
 int split_error_status(sht_plan *p);  // reads and clears the device error word (synchronous)
-// one block whose bounded wait runs out on purpose and sets the error word (synchronous)
-int wait_selftest(sht_plan *p, unsigned long long limit_ns);
+// one block each whose bounded wait runs out on purpose and sets the error word
+int launch_band_wait_selftest(const sht_plan *p, unsigned long long limit_ns, cudaStream_t s);
+int launch_split_wait_selftest(sht_plan *p, unsigned long long limit_ns, cudaStream_t s);
 // Reads and clears every device error word of the plan (synchronous).
 int device_error_status(sht_plan *p);
 

@@ -109,9 +109,12 @@ struct BandCtl {
   int *taken, *abort_flag, *err;
 };
 
-// Waits for a phase, for at most two seconds of wall time: then the error word
-// is set and every role of the block leaves its loop.
-__device__ __forceinline__ bool band_wait(const BandCtl &c, uint64_t *bar, uint32_t parity)
+constexpr uint64_t kBandWaitLimit = 2000000000ull;  // 2 s per bounded wait
+
+// Waits for a phase, for at most limit_ns of wall time: then the error word is
+// set and every role of the block leaves its loop.
+__device__ __forceinline__ bool band_wait(const BandCtl &c, uint64_t *bar, uint32_t parity,
+                                          uint64_t limit_ns = kBandWaitLimit)
 {
   const uint32_t addr = tc::smem_addr(bar);
   bool ok = true;
@@ -121,7 +124,7 @@ __device__ __forceinline__ bool band_wait(const BandCtl &c, uint64_t *bar, uint3
     if (*(volatile int *)c.abort_flag) { ok = false; break; }
     const uint64_t now = tc::globaltimer_ns();
     if (t0 == 0) t0 = now;
-    if (now - t0 > 2000000000ull) {
+    if (now - t0 > limit_ns) {
       *(volatile int *)c.abort_flag = 1;
       *(volatile int *)c.err = SHT_ERR_DEVICE_TIMEOUT;
       __threadfence_system();
@@ -216,7 +219,7 @@ __device__ void band_produce(const BandArgs &a, const CUtensorMap *map, char *sm
     const int last = g - 1 - (g - 1 - s) % NS;  // last stage issued to slot s
     const uint64_t t0 = tc::globaltimer_ns();
     while (!tc::mbar_try(tc::smem_addr(c.full + s), (last / NS) & 1))
-      if (tc::globaltimer_ns() - t0 > 2000000000ull) break;
+      if (tc::globaltimer_ns() - t0 > kBandWaitLimit) break;
   }
 }
 
@@ -438,6 +441,24 @@ __global__ void __launch_bounds__(32 * (W + 1) * TEAMS, MINB) k_leg_band(const _
   }
 }
 
+// The failure path of the waits above, run on purpose: the first warp waits on a
+// barrier that nothing arrives at, gives up after limit_ns, raises the abort flag
+// and records the timeout; the second, waiting on the same barrier with the full
+// limit, leaves on the flag.  No copies are in flight.
+__global__ void __launch_bounds__(64) k_band_wait_selftest(int *err, uint64_t limit_ns)
+{
+  __shared__ __align__(8) uint64_t bar;
+  __shared__ int words[2];
+  if (threadIdx.x == 0) {
+    tc::mbar_init(&bar, 1);
+    words[0] = words[1] = 0;
+    tc::mbar_fence_init();
+  }
+  __syncthreads();
+  const BandCtl c{&bar, &bar, nullptr, words, words + 1, err};
+  band_wait(c, &bar, 0, threadIdx.x < 32 ? limit_ns : kBandWaitLimit);
+}
+
 // 8 x 8 blocks from the row-major table: one thread per element
 __global__ void k_band_table(int N, int JH, int nlt, const double *__restrict__ P, const long long *__restrict__ poff,
                              const long long *__restrict__ boff, double *__restrict__ out)
@@ -491,6 +512,14 @@ static int take_error_word(int **out)
   }
   *out = words + taken++ % kWords;
   return SHT_OK;
+}
+
+int launch_band_wait_selftest(const sht_plan *p, unsigned long long limit_ns, cudaStream_t s)
+{
+  k_band_wait_selftest<<<1, 64, 0, s>>>(p->err_word, limit_ns);
+  count_launch();
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? SHT_OK : cuda_fail(e, "k_band_wait_selftest");
 }
 
 int band_error_status(sht_plan *p)

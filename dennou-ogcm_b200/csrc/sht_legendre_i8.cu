@@ -351,7 +351,7 @@ struct Ctl {
 
 // Bounded wait on a phase; false on timeout (which also raises the abort
 // flag and the error word) or when another role has aborted.
-__device__ bool wait_ph(const Ctl &c, int b, uint32_t parity)
+__device__ __forceinline__ bool wait_ph_for(const Ctl &c, int b, uint32_t parity, uint64_t limit_ns)
 {
   const uint32_t addr = tc::smem_addr(c.bar + b);
   if (tc::mbar_try(addr, parity)) return true;
@@ -361,13 +361,14 @@ __device__ bool wait_ph(const Ctl &c, int b, uint32_t parity)
     // 1 ms passes), so a waiting warp takes no issue slots from working ones
     if (tc::mbar_try_sleep(addr, parity, 1000000u)) return true;
     if (*c.abort_flag) return false;
-    if (tc::globaltimer_ns() - t0 > kWaitLimit) {
+    if (tc::globaltimer_ns() - t0 > limit_ns) {
       *c.abort_flag = 1;
       atomicExch(c.err, SHT_ERR_DEVICE_TIMEOUT);
       return false;
     }
   }
 }
+__device__ bool wait_ph(const Ctl &c, int b, uint32_t parity) { return wait_ph_for(c, b, parity, kWaitLimit); }
 // the same for a whole warp: lane 0 waits (acquiring the phase), and the
 // shuffle both gives every lane the outcome and orders the lanes' later
 // accesses after lane 0's acquire
@@ -1065,25 +1066,27 @@ int launch_leg_inv_split(sht_plan *p, const double2 *Sp, int ncol, double2 *F, c
   return launch_i8(p, true, Sp, ncol, F, s);
 }
 
-// The failure path of the bounded waits, run on purpose: one block waits on a
-// shared-memory barrier that nothing arrives at, through the same bounded
-// poll the split kernel uses, gives up after limit_ns and records the
-// timeout in the plan's error word as the split kernel does.  It holds no
-// TMEM and waits on nothing outside its own block.
-__global__ void __launch_bounds__(128) k_wait_selftest(int *err, unsigned long long limit_ns)
+// The failure path of the bounded waits, run on purpose: the first warp waits
+// on a barrier that nothing arrives at, gives up after limit_ns, raises the
+// abort flag and records the timeout; the second, waiting on the same barrier
+// with the full limit, leaves on the flag.  The block holds no TMEM and waits on
+// nothing outside itself.
+__global__ void __launch_bounds__(64) k_wait_selftest(int *err, unsigned long long limit_ns)
 {
   __shared__ __align__(8) uint64_t mbar;
+  __shared__ int abort_flag;
   if (threadIdx.x == 0) {
     tc::mbar_init(&mbar, 1);
+    abort_flag = 0;
     tc::mbar_fence_init();
   }
   __syncthreads();
-  const bool done = tc::mbar_wait(&mbar, 0, limit_ns);
-  if (!done && (threadIdx.x & 31) == 0) atomicExch(err, SHT_ERR_DEVICE_TIMEOUT);
-  __syncthreads();
+  const Ctl c{&mbar, &abort_flag, err};
+  if (threadIdx.x == 0) wait_ph_for(c, 0, 0, limit_ns);
+  if (threadIdx.x >= 32) warp_wait(c, 0, 0);
 }
 
-int wait_selftest(sht_plan *p, unsigned long long limit_ns)
+int launch_split_wait_selftest(sht_plan *p, unsigned long long limit_ns, cudaStream_t s)
 {
   if (!split_supported(p)) {
     set_error("device timeout self-test: this grid has no split-precision error word");
@@ -1091,10 +1094,9 @@ int wait_selftest(sht_plan *p, unsigned long long limit_ns)
   }
   int rc = build_i8_tables(p);
   if (rc) return rc;
-  k_wait_selftest<<<1, 128, 0, p->stream>>>(tables(p)->d_err, limit_ns);
+  k_wait_selftest<<<1, 64, 0, s>>>(tables(p)->d_err, limit_ns);
   count_launch();
   cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaStreamSynchronize(p->stream);
   return e == cudaSuccess ? SHT_OK : cuda_fail(e, "k_wait_selftest");
 }
 

@@ -201,26 +201,5 @@ __device__ __forceinline__ uint64_t globaltimer_ns()
   return t;
 }
 
-// Wait for the phase with parity `parity` to complete.  Gives up once
-// `limit_ns` of wall time has passed (try_wait itself may suspend for a
-// system-defined time per poll, so the bound is on time, not on polls) and
-// returns false; the caller records the timeout and unwinds.
-__device__ __forceinline__ bool mbar_wait(uint64_t *mbar, uint32_t parity, uint64_t limit_ns)
-{
-  const uint32_t a = smem_addr(mbar);
-  const uint64_t t0 = globaltimer_ns();
-  while (true) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(done)
-        : "r"(a), "r"(parity));
-    if (done) return true;
-    if (globaltimer_ns() - t0 > limit_ns) return false;
-  }
-}
-
 }  // namespace tc
 }  // namespace sht

@@ -147,15 +147,19 @@ SHT_API int sht_set_option(sht_plan *plan, int option, int value);
 SHT_API int sht_get_option(const sht_plan *plan, int option, int *value);
 
 /* Self-test of the device-side failure path: one block waits, through the
- * bounded wait the split-precision kernel uses, on a shared-memory barrier
+ * bounded wait of the split-precision kernel, on a shared-memory barrier
  * that nothing arrives at, gives up after limit_ms milliseconds (1..1000)
- * and records the timeout in the plan's device error word.  Returns what the
- * status check after a synchronous call then reports:
- * SHT_ERR_DEVICE_TIMEOUT when the bound and the error word work.  The word is
- * cleared and the plan stays usable.  No counterpart in the reference (its
- * failures abort through MessageNotify).  Grids outside the split kernel
- * return SHT_ERR_UNSUPPORTED_SIZE. */
+ * and records the timeout in the plan's error word of that kernel; then the
+ * same with the FP64 kernels' wait and word.  Returns what the status check
+ * after a synchronous call then reports: SHT_ERR_DEVICE_TIMEOUT when both
+ * bounds and both words work.  The words are cleared and the plan stays
+ * usable.  No counterpart in the reference (its failures abort through
+ * MessageNotify).  Grids outside the split kernel return
+ * SHT_ERR_UNSUPPORTED_SIZE.  The _dev form runs the FP64 kernels' wait alone on
+ * the plan's stream, like a device call that times out: it returns without
+ * waiting, and the timeout is reported where a device call's is. */
 SHT_API int sht_selftest_device_timeout(sht_plan *plan, int limit_ms);
+SHT_API int sht_selftest_device_timeout_dev(sht_plan *plan, int limit_ms);
 
 /* Stream for the *_dev calls (a cudaStream_t passed as void*; NULL = legacy
  * default stream), and a wait for all work on it. */
