@@ -77,11 +77,12 @@ cudaError_t kernel_setup(const void *kern, size_t smem, int threads, int *per_sm
 
 // The bounded device-side waits are those of the band kernels, whose error
 // word is host memory, and of the split-precision kernel, whose error word is
-// read only once its tables exist.
+// read only once its tables exist.  Both are read and cleared, so that a timeout
+// in one is not left to be reported for a later call.
 int device_error_status(sht_plan *p)
 {
-  const int rc = band_error_status(p);
-  return rc ? rc : split_error_status(p);
+  const int split = split_error_status(p), band = band_error_status(p);
+  return band ? band : split;
 }
 
 namespace {
@@ -1052,7 +1053,9 @@ int sht_selftest_device_timeout_dev(sht_plan *p, int limit_ms)
   std::lock_guard<std::mutex> lk(p->mtx);
   DeviceGuard g(p->device);
   if (!g.ok) { set_error("cudaSetDevice failed"); return SHT_ERR_CUDA; }
-  return launch_band_wait_selftest(p, (unsigned long long)limit_ms * 1000000ull, p->stream);
+  const unsigned long long ns = (unsigned long long)limit_ms * 1000000ull;
+  if (p->tc_tables && (rc = launch_split_wait_selftest(p, ns, p->stream))) return rc;
+  return launch_band_wait_selftest(p, ns, p->stream);
 }
 
 int sht_set_stream(sht_plan *p, void *stream)

@@ -155,8 +155,9 @@ SHT_API int sht_get_option(const sht_plan *plan, int option, int *value);
  * bounds and both words work.  The words are cleared and the plan stays
  * usable.  No counterpart in the reference (its failures abort through
  * MessageNotify).  Grids outside the split kernel return
- * SHT_ERR_UNSUPPORTED_SIZE.  The _dev form runs the FP64 kernels' wait alone on
- * the plan's stream, like a device call that times out: it returns without
+ * SHT_ERR_UNSUPPORTED_SIZE.  The _dev form runs the FP64 kernels' wait (after
+ * the split kernel's, on a plan that has made a split-precision call) on the
+ * plan's stream, like a device call that times out: it returns without
  * waiting, and the timeout is reported where a device call's is. */
 SHT_API int sht_selftest_device_timeout(sht_plan *plan, int limit_ms);
 SHT_API int sht_selftest_device_timeout_dev(sht_plan *plan, int limit_ms);

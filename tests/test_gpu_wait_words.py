@@ -54,3 +54,21 @@ def test_fp64_wait_on_the_plans_stream():
         assert np.array_equal(s.wa_xya(x), want)
     finally:
         s.final()
+
+
+def test_timeouts_in_both_words_are_reported_once():
+    P = pkg()
+    lib = P.load_library()
+    s = P.SpmlUtil(64, 32, 1, 21)
+    try:
+        x = np.random.default_rng(2).standard_normal((2, 32, 64))
+        want = s.wa_xya(x)
+        assert lib.sht_selftest_device_timeout(s._h, 1) == TIMEOUT  # builds the digit tables
+        t0 = time.perf_counter()
+        assert lib.sht_selftest_device_timeout_dev(s._h, 100) == 0
+        assert lib.sht_synchronize(s._h) == TIMEOUT
+        assert time.perf_counter() - t0 >= 0.2  # both waits ran
+        assert lib.sht_synchronize(s._h) == 0
+        assert np.array_equal(s.wa_xya(x), want)
+    finally:
+        s.final()
