@@ -666,6 +666,7 @@ void free_plan(sht_plan *p)
   if (p->copy_out) cudaStreamDestroy(p->copy_out);
   for (auto &ev : p->chunk_ev)
     if (ev) cudaEventDestroy(ev);
+  return_error_word(p);  // cudaFree above waited for the device
 }
 
 }  // namespace

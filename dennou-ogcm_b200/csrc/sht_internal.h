@@ -127,7 +127,7 @@ struct sht_plan_s {
   double *d_band_P = nullptr;
   long long *d_band_off = nullptr;
   sht::BandItem *d_band_items = nullptr;  // analysis items, then synthesis items
-  int *err_word = nullptr;  // host-mapped word their bounded waits report a timeout in
+  int *err_word = nullptr, *err_dev = nullptr;  // host word their bounded waits report a timeout in, its device address
   int n_band_f = 0, n_band_i = 0;
   int band_tf = 0, band_ti = 0;  // most 8-row tiles of an item
   // the last data tensor map of each direction: encoding one costs a launch
@@ -207,6 +207,7 @@ int launch_fft_inv(const sht_plan *p, const double2 *F, int ncolF, int colF0, in
 int plan_band_items(sht_plan *p, std::vector<long long> &boff, std::vector<BandItem> &items);
 int build_band_table(sht_plan *p);
 int band_error_status(sht_plan *p);  // reads and clears the plan's error word (after a synchronisation)
+void return_error_word(sht_plan *p);  // once none of the plan's kernels can run any more
 int launch_leg_fwd_fp64(const sht_plan *p, const double2 *F, int ncol, double2 *S, cudaStream_t s);
 int launch_leg_inv_fp64(const sht_plan *p, const double2 *S, int ncol, double2 *F, cudaStream_t s);
 

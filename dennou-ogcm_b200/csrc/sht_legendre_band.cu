@@ -55,6 +55,8 @@
 #include "sht_tc.cuh"
 
 #include <algorithm>
+#include <cstdlib>
+#include <mutex>
 
 namespace sht {
 
@@ -77,7 +79,7 @@ struct BandArgs {
   int lgcw;           // log2 CW
   int J, JH, ncol;
   int drop;           // the Fourier lines are read by one item only: drop them from L2
-  int *err;           // host-mapped error word of the plan
+  int *err;           // the plan's error word (page-locked host memory)
 };
 
 // k-th unit of block b: the largest-first list is dealt out to the G blocks
@@ -492,31 +494,81 @@ constexpr int kItemCap = 8;
 
 }  // namespace
 
-// The plans' error words: one page-locked array that every device can write,
-// allocated with the first plan and kept (4 KB); plans take its words in turn,
-// so past 1024 plans two may share one and either may report the other's
-// timeout.
-static int take_error_word(int **out)
+// The plans' error words.  A page of them is ordinary memory of this process,
+// never freed and registered with the plans' device, so that the host may read a
+// word whatever became of the context it was registered in; a page whose
+// registration went with a device reset is registered again for the next plan.
+// A word belongs to one live plan, is zero when it is handed out, and comes back
+// with sht_final.
+namespace {
+
+struct ErrorPage {
+  int device;
+  int *words;
+  std::vector<int> unused;
+};
+constexpr int kPageWords = 1024;
+std::mutex g_error_mutex;
+std::vector<ErrorPage> &error_pages()
 {
-  constexpr int kWords = 1024;
-  static std::mutex mu;
-  static int *words = nullptr;
-  static unsigned taken = 0;
-  std::lock_guard<std::mutex> lk(mu);
-  if (!words) {
-    void *h = nullptr;
-    cudaError_t e = cudaHostAlloc(&h, sizeof(int) * kWords, cudaHostAllocMapped | cudaHostAllocPortable);
-    if (e != cudaSuccess) return cuda_fail(e, "cudaHostAlloc(error words)");
-    words = static_cast<int *>(h);
-    std::fill(words, words + kWords, 0);
+  static auto *pages = new std::vector<ErrorPage>;  // outlives plans that are finalised at exit
+  return *pages;
+}
+
+// the page's address on its device (current), registering it where it is not
+cudaError_t page_address(const ErrorPage &g, int **dev)
+{
+  cudaPointerAttributes at;
+  cudaError_t e = cudaPointerGetAttributes(&at, g.words);
+  if (e != cudaSuccess || at.type == cudaMemoryTypeUnregistered) {
+    cudaGetLastError();
+    if ((e = cudaHostRegister(g.words, sizeof(int) * kPageWords, cudaHostRegisterMapped)) != cudaSuccess) return e;
   }
-  *out = words + taken++ % kWords;
+  void *d = nullptr;
+  e = cudaHostGetDevicePointer(&d, g.words, 0);
+  *dev = static_cast<int *>(d);
+  return e;
+}
+
+int take_error_word(sht_plan *p)
+{
+  std::lock_guard<std::mutex> lk(g_error_mutex);
+  auto &pages = error_pages();
+  ErrorPage *g = nullptr;
+  for (ErrorPage &c : pages)
+    if (!g && c.device == p->device && !c.unused.empty()) g = &c;
+  if (!g) {
+    int *w = static_cast<int *>(std::aligned_alloc(4096, sizeof(int) * kPageWords));
+    if (!w) { set_error("error words: host allocation failed"); return SHT_ERR_ALLOC; }
+    pages.push_back({p->device, w, {}});
+    g = &pages.back();
+    for (int k = kPageWords; k-- > 0;) g->unused.push_back(k);
+  }
+  int *dev = nullptr;
+  const cudaError_t e = page_address(*g, &dev);
+  if (e != cudaSuccess) return cuda_fail(e, "error words");
+  const int k = g->unused.back();
+  g->unused.pop_back();
+  p->err_word = g->words + k;
+  p->err_dev = dev + k;
+  *(volatile int *)p->err_word = 0;
   return SHT_OK;
+}
+
+}  // namespace
+
+void return_error_word(sht_plan *p)
+{
+  if (!p->err_word) return;
+  std::lock_guard<std::mutex> lk(g_error_mutex);
+  for (ErrorPage &g : error_pages())
+    if (p->err_word >= g.words && p->err_word < g.words + kPageWords) g.unused.push_back((int)(p->err_word - g.words));
+  p->err_word = p->err_dev = nullptr;
 }
 
 int launch_band_wait_selftest(const sht_plan *p, unsigned long long limit_ns, cudaStream_t s)
 {
-  k_band_wait_selftest<<<1, 64, 0, s>>>(p->err_word, limit_ns);
+  k_band_wait_selftest<<<1, 64, 0, s>>>(p->err_dev, limit_ns);
   count_launch();
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? SHT_OK : cuda_fail(e, "k_band_wait_selftest");
@@ -534,7 +586,7 @@ int band_error_status(sht_plan *p)
 // is the block count) and the item lists of both directions, largest first.
 int plan_band_items(sht_plan *p, std::vector<long long> &boff, std::vector<BandItem> &items)
 {
-  const int rc = take_error_word(&p->err_word);
+  const int rc = take_error_word(p);
   if (rc) return rc;
   const int N = p->N, M = p->M, nlt = (p->JH + 7) / 8;
   auto count = [&](int m, int par) { const int R = N + 2 - m; return par ? R / 2 : (R + 1) / 2; };
@@ -671,7 +723,7 @@ int launch_band(const sht_plan *p, BandArgs a, cudaStream_t s)
   a.P = p->d_band_P;
   a.items = p->d_band_items + (INV ? p->n_band_f : 0);
   a.J = p->J; a.JH = p->JH;
-  a.err = p->err_word;
+  a.err = p->err_dev;
   const int tm = INV ? p->band_ti : p->band_tf;
   // One block of three teams, or three blocks of one.  The teams share the SM's
   // units, which pays where a unit is long (analysis / synthesis, T170, 720:
