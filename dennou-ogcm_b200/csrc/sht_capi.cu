@@ -85,6 +85,16 @@ int device_error_status(sht_plan *p)
   return band ? band : split;
 }
 
+// A device call that timed out has returned SHT_OK before its kernels ran: the
+// next call on the plan reports what its word says by now, and does not run (the
+// split kernel's word is device memory and is read by synchronous calls only).
+int earlier_timeout_status(sht_plan *p)
+{
+  const int rc = band_error_status(p);
+  if (rc) set_error("an earlier call on this plan timed out and left its results incomplete (this call did not run)");
+  return rc;
+}
+
 namespace {
 
 struct DeviceGuard {
@@ -385,6 +395,7 @@ int api_dev(sht_plan *p, int op, const double *i0, const double *i1, int nb, dou
   std::lock_guard<std::mutex> lk(p->mtx);
   DeviceGuard g(p->device);
   if (!g.ok) { set_error("cudaSetDevice failed"); return SHT_ERR_CUDA; }
+  if ((rc = earlier_timeout_status(p))) return rc;
   rc = run_dev(p, op, i0, i1, nb, o0, o1, i2);
   if (!rc) finish_timing(p, !shape_of(op).out_grid);
   return rc;
@@ -498,6 +509,7 @@ int api_host(sht_plan *p, int op, const double *i0, const double *i1, int nb, do
   std::lock_guard<std::mutex> lk(p->mtx);
   DeviceGuard g(p->device);
   if (!g.ok) { set_error("cudaSetDevice failed"); return SHT_ERR_CUDA; }
+  if ((rc = earlier_timeout_status(p))) return rc;
   return host_call(p, op, i0, i1, nb, o0, o1, i2);
 }
 
@@ -756,7 +768,8 @@ int strided_call(sht_plan *p, bool analysis, const double *g_in, double *g_out, 
   DeviceGuard guard(p->device);
   if (!guard.ok) { set_error("cudaSetDevice failed"); return SHT_ERR_CUDA; }
   PrecisionScope ps(p, mode);
-  int rc;
+  int rc = earlier_timeout_status(p);
+  if (rc) return rc;
   if (ldi == p->I && ldj == p->J && ldw == p->L) {  // contiguous: the ordinary call
     const int op = analysis ? OP_W_XY : OP_XY_W;
     const double *in = analysis ? g_in : w_in;
@@ -1175,6 +1188,7 @@ static int uv_fma_impl(sht_plan *p, const double *x1, const double *x2, const do
   std::lock_guard<std::mutex> lk(p->mtx);
   DeviceGuard g(p->device);
   if (!g.ok) { set_error("cudaSetDevice failed"); return SHT_ERR_CUDA; }
+  if ((rc = earlier_timeout_status(p))) return rc;
   if (!host) {
     rc = run_analysis(p, PACK_VORDIV, RS_FWD_INVCOS, x1, x2, nb, vor, div, q, z1, z2);
     if (!rc) finish_timing(p, true);
@@ -1259,6 +1273,7 @@ static int diffuse_impl(sht_plan *p, const double *w, int nb, const double *coef
   std::lock_guard<std::mutex> lk(p->mtx);
   DeviceGuard g(p->device);
   if (!g.ok) { set_error("cudaSetDevice failed"); return SHT_ERR_CUDA; }
+  if ((rc = earlier_timeout_status(p))) return rc;
   cudaStream_t s = p->stream;
   cudaError_t e;
   if (!host) return launch_diffuse(p, w, nb, coef, dt, filter, out, s);
@@ -1292,6 +1307,7 @@ int sht_wa_sub_filter_dev(sht_plan *p, double *wa, const double *wb, int nb, con
   std::lock_guard<std::mutex> lk(p->mtx);
   DeviceGuard g(p->device);
   if (!g.ok) { set_error("cudaSetDevice failed"); return SHT_ERR_CUDA; }
+  if ((rc = earlier_timeout_status(p))) return rc;
   return launch_sub_filter(p, wa, wb, nb, filter, p->stream);
 }
 
@@ -1304,6 +1320,7 @@ int sht_wa_sub_lapla_dev(sht_plan *p, double *wa, double *wneg, const double *wc
   std::lock_guard<std::mutex> lk(p->mtx);
   DeviceGuard g(p->device);
   if (!g.ok) { set_error("cudaSetDevice failed"); return SHT_ERR_CUDA; }
+  if ((rc = earlier_timeout_status(p))) return rc;
   return launch_sub_lapla(p, wa, wneg, wc, nb, p->stream);
 }
 
@@ -1317,6 +1334,7 @@ int sht_roundtrip_diffuse_dev(sht_plan *p, double *xya, int nb, const double *co
   std::lock_guard<std::mutex> lk(p->mtx);
   DeviceGuard g(p->device);
   if (!g.ok) { set_error("cudaSetDevice failed"); return SHT_ERR_CUDA; }
+  if ((rc = earlier_timeout_status(p))) return rc;
   Workspace ws{};
   if ((rc = ensure_ws(p, nb, nb, &ws))) return rc;
   if ((rc = run_analysis(p, PACK_PLAIN, RS_FWD_PLAIN, xya, nullptr, nb, ws.W, nullptr))) return rc;

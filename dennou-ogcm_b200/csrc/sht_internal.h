@@ -261,6 +261,8 @@ int launch_band_wait_selftest(const sht_plan *p, unsigned long long limit_ns, cu
 int launch_split_wait_selftest(sht_plan *p, unsigned long long limit_ns, cudaStream_t s);
 // Reads and clears every device error word of the plan (synchronous).
 int device_error_status(sht_plan *p);
+// What the host-readable one says of calls that have finished (no waiting).
+int earlier_timeout_status(sht_plan *p);
 
 // --- column-table pipelines (sht_capi.cu), used by the multi-instance batches
 // F holds (N+1) J ncol complex values, S holds R ncol; the plan mutex is held

@@ -433,6 +433,8 @@ int sht_multi_run(sht_multi *m, int what)
   if (what < SHT_MULTI_SYNTHESIS || what > SHT_MULTI_ROUND_TRIP) { set_error("multi: unknown step"); return SHT_ERR_INVALID_ARG; }
   std::lock_guard<std::mutex> lk(m->mtx);
   if (!m->built) { set_error("multi: call sht_multi_build first"); return SHT_ERR_NOT_INITIALIZED; }
+  for (Group &g : m->groups)
+    if (const int rc = earlier_timeout_status(g.plan)) return rc;
   DevGuard g(m->device);
   if (!g.ok) { set_error("cudaSetDevice failed"); return SHT_ERR_CUDA; }
   if (m->use_graph) {

@@ -89,6 +89,7 @@ extern "C" SHT_API int sht_wa_xya_dev_noalloc(sht_plan *p, const double *xya, in
     return SHT_ERR_TOO_LARGE;
   }
   std::lock_guard<std::mutex> lk(p->mtx);
+  if (const int late = earlier_timeout_status(p)) return late;
   if (use_split(p, true) && !p->tc_tables) {
     // the split kernel's digit tables are allocated by the first split-precision
     // transform of a plan; this entry point must not be the one to do it

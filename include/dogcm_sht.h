@@ -25,7 +25,11 @@
  *  - Functions without a suffix take HOST pointers and return when the
  *    results are in host memory.  The *_dev variants take DEVICE pointers and
  *    are ordered on the plan's stream (sht_set_stream).  They return once the
- *    work is enqueued.
+ *    work is enqueued, so a device-side timeout of one (a bounded wait of 2 s
+ *    that ran out: its results are incomplete) cannot be in its own status.
+ *    sht_synchronize reports it (SHT_ERR_DEVICE_TIMEOUT); so does the next call
+ *    on the plan after it happened, which then does not run (FP64; a timeout in
+ *    split precision is reported by sht_synchronize and by host calls).
  *  - Calls on one plan are serialised internally: the plan owns its device
  *    workspace.  Different plans may be used from different host threads.
  *  - There is no CPU fallback.  Without a usable CUDA device every compute

@@ -72,3 +72,52 @@ def test_timeouts_in_both_words_are_reported_once():
         assert np.array_equal(s.wa_xya(x), want)
     finally:
         s.final()
+
+
+def test_next_call_reports_a_device_calls_timeout():
+    """A device call that times out has returned 0 by then: whichever call comes
+    next on the plan returns the status, without running, and the one after it runs."""
+    import torch
+
+    P = pkg()
+    lib = P.load_library()
+    im, jm, nm, nb = 64, 32, 21, 2
+    s, other = P.SpmlUtil(im, jm, 1, nm), P.SpmlUtil(im, jm, 1, nm)
+    try:
+        g = torch.Generator(device="cuda")
+        g.manual_seed(5)
+        x, y, q = (torch.randn(nb, jm, im, generator=g, device="cuda", dtype=torch.float64) for _ in range(3))
+        w, v = (torch.randn(nb, s.lm, generator=g, device="cuda", dtype=torch.float64) for _ in range(2))
+        c = torch.rand(s.lm, generator=g, device="cuda", dtype=torch.float64)
+        halo = torch.zeros(nb, jm + 2, im + 2, device="cuda", dtype=torch.float64)
+        xh, wh = x.cpu().numpy(), w.cpu().numpy()
+        out = torch.empty_like(w)
+        m = P.MultiTransform()
+        m.add(s, w.clone(), x.clone())
+        m.build()
+
+        def noalloc():
+            st = lib.sht_wa_xya_dev_noalloc(s._h, x.data_ptr(), nb, out.data_ptr())
+            if st:
+                raise P.SpmlError(st, "noalloc", lib.sht_last_error().decode())
+
+        lib.sht_wa_xya_dev_noalloc.argtypes = lib.sht_wa_xya_dev.argtypes
+        calls = [lambda: s.w_xy(x), lambda: s.xy_w(w), lambda: s.calc_UVCosLat2VorDiv_fma(x, y, q), lambda: s.diffuse(w, c, 0.5),
+                 lambda: s._sub_filter(w.clone(), v, c), lambda: s._sub_lapla(w.clone(), v.clone(), w),
+                 lambda: s.analysis(halo, 1, 1), lambda: s.synthesis(w, halo, 1, 1), lambda: s.roundtrip_diffuse_(x.clone()),
+                 noalloc, m.run, lambda: s.w_xy(xh), lambda: s.xy_w(wh), lambda: s.diffuse(wh, c.cpu().numpy(), 0.5)]
+        for k, call in enumerate(calls):
+            call()
+            assert lib.sht_selftest_device_timeout_dev(s._h, 1) == 0
+            torch.cuda.synchronize()
+            other.w_xy(x)  # another plan is not concerned
+            with pytest.raises(P.SpmlError) as e:
+                call()
+            assert e.value.status == TIMEOUT and "earlier call" in str(e.value), k
+            call()
+            assert lib.sht_synchronize(s._h) == 0
+        assert torch.equal(s.w_xy(x), other.w_xy(x))
+        m.close()
+    finally:
+        s.final()
+        other.final()
