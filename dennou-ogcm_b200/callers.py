@@ -21,8 +21,10 @@ from .spmlutil import SpmlUtil
 
 def _spectra(sp, *ws):
     """Whether ws are results of this package's plan that the fused tails may
-    overwrite: plain CUDA float64 (K, lm) tensors."""
-    if not isinstance(sp, SpmlUtil):
+    overwrite: plain CUDA float64 (K, lm) tensors of a SpmlUtil itself, whose
+    transforms hand out new tensors (a subclass may keep them, or have its own
+    Laplacian)."""
+    if type(sp) is not SpmlUtil:
         return False
     import torch
 
