@@ -432,9 +432,7 @@ int host_graph_call(sht_plan *p, int op, int nb, Enqueue &&enqueue)
   }
   HostGraph *g = nullptr;
   for (HostGraph &c : gs)
-    if (c.op == op && c.nb == nb && c.precision == p->precision && c.leg_kernel == p->leg_kernel &&
-        c.leg_tile == p->leg_tile)
-      g = &c;
+    if (c.op == op && c.nb == nb && c.precision == p->precision && c.small == wants_small(p)) g = &c;
   cudaError_t e;
   if (g && g->exec) {
     if ((e = cudaGraphLaunch(g->exec, s)) != cudaSuccess) return cuda_fail(e, "graph launch");
@@ -448,7 +446,7 @@ int host_graph_call(sht_plan *p, int op, int nb, Enqueue &&enqueue)
         gs.erase(gs.begin());
       }
       HostGraph n;
-      n.op = op; n.nb = nb; n.precision = p->precision; n.leg_kernel = p->leg_kernel; n.leg_tile = p->leg_tile;
+      n.op = op; n.nb = nb; n.precision = p->precision; n.small = wants_small(p);
       n.gen = p->buf_gen;
       gs.push_back(n);
     }
@@ -481,9 +479,7 @@ int host_graph_call(sht_plan *p, int op, int nb, Enqueue &&enqueue)
   // g may have moved if the list changed; find the entry again
   g = nullptr;
   for (HostGraph &c : gs)
-    if (c.op == op && c.nb == nb && c.precision == p->precision && c.leg_kernel == p->leg_kernel &&
-        c.leg_tile == p->leg_tile)
-      g = &c;
+    if (c.op == op && c.nb == nb && c.precision == p->precision && c.small == wants_small(p)) g = &c;
   if (rc != SHT_OK || e != cudaSuccess || !exec) {
     cudaGetLastError();
     if (exec) cudaGraphExecDestroy(exec);

@@ -66,7 +66,8 @@ struct Timing {
 // Every pointer in it is a plan buffer, so it replays for any caller arrays
 // of the same operator and size until a buffer is reallocated (buf_gen).
 struct HostGraph {
-  int op = -1, nb = 0, precision = 0, leg_kernel = 0, leg_tile = 0;
+  int op = -1, nb = 0, precision = 0;
+  bool small = false;              // captured with the single-kernel small-grid transform chosen
   unsigned long long gen = 0;
   cudaGraphExec_t exec = nullptr;  // null after the first call, or when not capturable
   bool failed = false;             // capture was refused: run this call uncaptured
@@ -238,10 +239,10 @@ inline bool use_split(const sht_plan *p, bool analysis)
 // im = 32 (16 complex points per row), the only size where it measured
 // faster than the batched kernels (T10, 480 field-levels: round trip 26
 // against 37 us); in FP64 only (split precision keeps the batched path)
+inline bool wants_small(const sht_plan *p) { return p->leg_kernel == 4 || (p->leg_kernel == 0 && p->NC == 16); }
 inline bool use_small(const sht_plan *p, bool analysis)
 {
-  const bool want = p->leg_kernel == 4 || (p->leg_kernel == 0 && p->NC == 16);
-  return want && !use_split(p, analysis) && small_supported(p);
+  return wants_small(p) && !use_split(p, analysis) && small_supported(p);
 }
 
 // SMs a plan's persistent kernels size their grids for
