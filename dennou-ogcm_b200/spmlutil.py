@@ -165,7 +165,9 @@ def _torch():
 
 def _raw_stream():
     """Device index -> handle of torch's current stream (0 for the default one)."""
-    return _torch()._C._cuda_getCurrentRawStream
+    torch = _torch()
+    # torch's own short cut, where this torch has it: no Stream object
+    return getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda dev: torch.cuda.current_stream(dev).cuda_stream)
 
 
 def _is_torch_cuda(x) -> bool:
