@@ -559,11 +559,18 @@ __device__ __forceinline__ void ldg32(const double2 *p, double2 &x, double2 &y)
 // largest value alone, and their digits meet zero table digits or columns that
 // are not stored.  Unconditional loads stay one batch in flight; guarded ones
 // were compiled into a chain (16 loads took 16 latencies).
-template <bool INV, int NV>
+// SHORT: analyses of fewer latitudes than a chunk, where a thread wholly past K
+// skips its batch (three threads of four at T21; with their repeated loads T21,
+// 480: 15.4 -> 17.0 us, 16 x 8 points, 200: 8.7 -> 9.8).  The same test in the
+// other analyses, where it is never true, took T170, 240: 133 -> 137 us.
+template <bool INV, int NV, bool SHORT = false>
 __device__ __forceinline__ void loadn(const I8Args &a, const Unit &u, int col, int k0, double2 (&x)[NV])
 {
   col = min(col, a.ncol - 1);
-  if (!INV) {
+  if (SHORT && k0 >= u.K) {
+#pragma unroll
+    for (int i = 0; i < NV; ++i) x[i] = make_double2(0.0, 0.0);
+  } else if (!INV) {
     const double2 *src = a.F + ((long long)u.m * a.ncol + col) * a.J + u.p * a.JH;
     if (u.K % 2 == 0) {
 #pragma unroll
@@ -596,7 +603,7 @@ __device__ __forceinline__ void hmaxn(const double2 (&y)[NV], int &r, int &im)
   }
 }
 
-template <bool INV, bool CACHE>
+template <bool INV, bool CACHE, bool SHORT>
 __device__ void role_convert(const I8Args &a, const Ctl &c, unsigned char *As, int *exps, const Lut &t, Unit u, bool have, int g1)
 {
   using R = Roles<INV>;
@@ -677,12 +684,12 @@ __device__ void role_convert(const I8Args &a, const Ctl &c, unsigned char *As, i
 #pragma unroll 1
           for (int i0 = 0; i0 < 16; i0 += PB) {
             double2 y[PB];
-            loadn<INV, PB>(a, u, col, kc * kKC + 16 * q + i0, y);
+            loadn<INV, PB, SHORT>(a, u, col, kc * kKC + 16 * q + i0, y);
             hmaxn<PB>(y, mr, mi);
           }
       }
       double2 x[16];
-      loadn<INV, 16>(a, u, col, k0, x);
+      loadn<INV, 16, SHORT>(a, u, col, k0, x);
       if (!SCAN && first) {
         hmax(x, mr, mi);
         mr = max(mr, __shfl_xor_sync(0xffffffffu, mr, 8));
@@ -851,7 +858,7 @@ __device__ void role_epilogue(const I8Args &a, const Ctl &c, const int *exps, ui
   }
 }
 
-template <bool INV, bool CACHE>
+template <bool INV, bool CACHE, bool SHORT = false>
 __global__ void __launch_bounds__(threads_of(scan_of(INV, CACHE)), 1) k_leg_i8(I8Args a)
 {
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -917,7 +924,7 @@ __global__ void __launch_bounds__(threads_of(scan_of(INV, CACHE)), 1) k_leg_i8(I
   } else if (warp == 1) {
     if (lane == 0) role_mma<INV, CACHE>(a, c, tc::smem_addr(As), tc::smem_addr(Ps), tbase, t, u, have, g1);
   } else if (warp < Roles<INV>::kEpi0) {
-    role_convert<INV, CACHE>(a, c, As, exps, t, u, have, g1);
+    role_convert<INV, CACHE, SHORT>(a, c, As, exps, t, u, have, g1);
   } else if (warp < Roles<INV>::kScan0) {
     role_epilogue<INV, CACHE>(a, c, exps, tbase, t, u, have, g1);
   } else if constexpr (scan_of(INV, CACHE)) {
@@ -1031,9 +1038,10 @@ int launch_i8(sht_plan *p, bool inverse, const double2 *in, int ncol, double2 *o
   a.per_cta = (a.nsub + slots - 1) / slots;
   const int grid = (a.nsub + a.per_cta - 1) / a.per_cta;
   // the digit-cache instance where some sub-item has more than two output
-  // segments (T170 and up), the plain one elsewhere
+  // segments (T170 and up), the plain ones elsewhere
   auto kern = inverse ? (a.scr ? k_leg_i8<true, true> : k_leg_i8<true, false>)
-                      : (a.scr ? k_leg_i8<false, true> : k_leg_i8<false, false>);
+            : a.scr   ? k_leg_i8<false, true>
+                      : (p->JH < kKC ? k_leg_i8<false, false, true> : k_leg_i8<false, false>);
   const size_t smem = kSmemFixed + lut_bytes(p->N, p->n_pairs);
   if (smem > 227 * 1024) {
     set_error("split precision: the truncation's lookup tables do not fit beside the stages");
