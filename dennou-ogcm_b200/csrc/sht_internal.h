@@ -83,6 +83,15 @@ struct alignas(16) BandItem {
   int row, cnt;
 };
 
+// The blocked Legendre table (sht_legendre_band.cu): element (k, jh) of a band
+// and parity whose blocks begin at block blk and lie in rows of nrt row tiles --
+// k-th degree of the parity, latitude jh.
+__host__ __device__ inline long long band_at(long long blk, int nrt, int k, int jh)
+{
+  const int d = k & 7;
+  return (blk + (long long)(jh >> 3) * nrt + (k >> 3)) * 64 + 8 * d + ((jh & 7) ^ (4 * ((d >> 1) & 1)));
+}
+
 }  // namespace sht
 
 struct sht_plan_s {
@@ -109,8 +118,7 @@ struct sht_plan_s {
   // device tables, all in one allocation
   void *d_tables = nullptr;
   double *d_mu = nullptr, *d_wgt = nullptr, *d_rowscale = nullptr;
-  double *d_P = nullptr;
-  long long *d_poff = nullptr;
+  double *d_P = nullptr;    // row-major Legendre table, where the small-grid kernel takes the plan
   int *d_rowoff = nullptr;
   double *d_eps = nullptr;  // [m][n], n = 0..N+2
   double2 *d_tw = nullptr;  // exp(-2 pi i k / NC), k < NC
@@ -206,7 +214,6 @@ int launch_fft_inv(const sht_plan *p, const double2 *F, int ncolF, int colF0, in
 // --- Legendre contraction, FP64: one band and parity per block, any grid
 // (sht_legendre_band.cu)
 int plan_band_items(sht_plan *p, std::vector<long long> &boff, std::vector<BandItem> &items);
-int build_band_table(sht_plan *p);
 int band_error_status(sht_plan *p);  // reads and clears the plan's error word (after a synchronisation)
 void return_error_word(sht_plan *p);  // once none of the plan's kernels can run any more
 int launch_leg_fwd_fp64(const sht_plan *p, const double2 *F, int ncol, double2 *S, cudaStream_t s);

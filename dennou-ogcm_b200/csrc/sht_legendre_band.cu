@@ -461,22 +461,6 @@ __global__ void __launch_bounds__(64) k_band_wait_selftest(int *err, uint64_t li
   band_wait(c, &bar, 0, threadIdx.x < 32 ? limit_ns : kBandWaitLimit);
 }
 
-// 8 x 8 blocks from the row-major table: one thread per element
-__global__ void k_band_table(int N, int JH, int nlt, const double *__restrict__ P, const long long *__restrict__ poff,
-                             const long long *__restrict__ boff, double *__restrict__ out)
-{
-  const int m = blockIdx.y >> 1, par = blockIdx.y & 1;
-  const int R = N + 2 - m, cnt = par ? R / 2 : (R + 1) / 2, nrt = (cnt + 7) >> 3;
-  const long long total = (long long)nlt * nrt * 64;
-  double *o = out + boff[2 * m + par] * 64;
-  for (long long x = blockIdx.x * (long long)blockDim.x + threadIdx.x; x < total; x += (long long)gridDim.x * blockDim.x) {
-    const int e = (int)(x & 63), d = e >> 3, l = (e & 7) ^ (4 * ((d >> 1) & 1));
-    const long long b = x >> 6;
-    const int lt = (int)(b / nrt), k = 8 * (int)(b - (long long)lt * nrt) + d, jh = 8 * lt + l;
-    o[x] = (k < cnt && jh < JH) ? P[poff[m] + (long long)(2 * k + par) * JH + jh] : 0.0;
-  }
-}
-
 int max_row_tiles(int N) { return ((N + 3) / 2 + 7) / 8; }
 
 // row tiles per item: the tiles of the largest band split evenly into items
@@ -613,18 +597,6 @@ int plan_band_items(sht_plan *p, std::vector<long long> &boff, std::vector<BandI
   p->n_band_i = (int)inv.size();
   items.insert(items.end(), inv.begin(), inv.end());
   return SHT_OK;
-}
-
-// Fills the blocked table from the row-major one (on the plan's stream).
-int build_band_table(sht_plan *p)
-{
-  const int nlt = (p->JH + 7) / 8;
-  const long long most = (long long)nlt * max_row_tiles(p->N) * 64;
-  k_band_table<<<dim3((unsigned)std::min<long long>((most + 255) / 256, 64), 2 * p->M), 256, 0, p->stream>>>(
-      p->N, p->JH, nlt, p->d_P, p->d_poff, p->d_band_off, p->d_band_P);
-  count_launch();
-  const cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? SHT_OK : cuda_fail(e, "k_band_table");
 }
 
 namespace {

@@ -150,7 +150,7 @@ I8Tables *tables(sht_plan *p) { return static_cast<I8Tables *>(p->tc_tables); }
 // over the degrees of parity p.  Layout per (m, p): K chunk, segment, digit,
 // then a canonical tile of npad rows x 64 bytes.
 template <bool INV>
-__global__ void k_i8_table(int N, int JH, const double *__restrict__ P, const long long *__restrict__ poff,
+__global__ void k_i8_table(int N, int JH, const double *__restrict__ P, const long long *__restrict__ boff,
                            uint8_t *tab, const long long *__restrict__ toff, double *tfac, const int *__restrict__ teoff)
 {
   const int mp = blockIdx.y, m = mp >> 1, p = mp & 1;
@@ -161,10 +161,9 @@ __global__ void k_i8_table(int N, int JH, const double *__restrict__ P, const lo
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= rows * nk16) return;
   const int r = idx / nk16, k16 = idx - r * nk16;
-  const double *base = P + poff[m];
-  auto val = [&](int k) -> double {
-    return INV ? base[(long long)(p + 2 * k) * JH + r] : base[(long long)(p + 2 * r) * JH + k];
-  };
+  const long long blk = boff[mp];
+  const int nrt = (Rp + 7) >> 3;
+  auto val = [&](int k) -> double { return P[INV ? band_at(blk, nrt, k, r) : band_at(blk, nrt, r, k)]; };
   double mx = 0.0;
   for (int k = 0; k < K; ++k) mx = fmax(mx, fabs(val(k)));
   const int e = i8::exp_of(mx);
@@ -1002,14 +1001,14 @@ int build_i8_tables(sht_plan *p)
   if ((e = cudaMemsetAsync(t->d_err, 0, sizeof(int), s)) != cudaSuccess) return fail(e, "split table upload");
   {
     const int maxrows = (N + 3) / 2, nk16 = (JH + 15) / 16;
-    dim3 g((maxrows * nk16 + 127) / 128, nmp);
-    k_i8_table<false><<<g, 128, 0, s>>>(N, JH, p->d_P, p->d_poff, t->tab[0], t->toff[0], t->tfac[0], t->teoff[0]);
+    dim3 g((maxrows * nk16 + 127) / 128, 2 * p->M);
+    k_i8_table<false><<<g, 128, 0, s>>>(N, JH, p->d_band_P, p->d_band_off, t->tab[0], t->toff[0], t->tfac[0], t->teoff[0]);
     count_launch();
   }
   {
     const int nk16 = ((N + 3) / 2 + 15) / 16;
-    dim3 g((JH * nk16 + 127) / 128, nmp);
-    k_i8_table<true><<<g, 128, 0, s>>>(N, JH, p->d_P, p->d_poff, t->tab[1], t->toff[1], t->tfac[1], t->teoff[1]);
+    dim3 g((JH * nk16 + 127) / 128, 2 * p->M);
+    k_i8_table<true><<<g, 128, 0, s>>>(N, JH, p->d_band_P, p->d_band_off, t->tab[1], t->toff[1], t->tfac[1], t->teoff[1]);
     count_launch();
   }
   if ((e = cudaGetLastError()) != cudaSuccess || (e = cudaStreamSynchronize(s)) != cudaSuccess) return fail(e, "split table build");

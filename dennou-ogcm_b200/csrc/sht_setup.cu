@@ -54,27 +54,43 @@ __global__ void k_gauss_nodes(int J, double *mu, double *wgt)
 
 // Pbar_n^m(mu_j) for the northern rows, one thread per (m, jh):
 //   Pbar_m^m = prod_{k<=m} sqrt((2k+1)/(2k)) (1-mu^2)^{m/2}
-//   Pbar_{n+1}^m = (mu Pbar_n^m - eps_n^m Pbar_{n-1}^m) / eps_{n+1}^m.
-__global__ void k_legendre_table(int N, int J, int JH, const double *__restrict__ mu,
-                                 const double *__restrict__ eps, const long long *__restrict__ poff,
-                                 double *__restrict__ P)
+//   Pbar_{n+1}^m = (mu Pbar_n^m - eps_n^m Pbar_{n-1}^m) / eps_{n+1}^m,
+// into the blocked table (zeros in the blocks' degrees and latitudes past the
+// last) and, where a plan's small-grid kernel reads it, the row-major one: rows
+// of JH latitudes in internal-row order.  Writing the blocks from a row-major
+// table kept both on every plan: T341 248 MB and 5.6 ms of set-up, 128 MB and
+// 5.2 ms with this (4.3 and 4.2 ms with one row-major table and this, elsewhere).
+__global__ void k_legendre_table(int N, int J, int JH, const double *__restrict__ mu, const double *__restrict__ eps,
+                                 const long long *__restrict__ boff, double *__restrict__ blocked,
+                                 double *__restrict__ rows)
 {
   const int jh = blockIdx.x * blockDim.x + threadIdx.x;
   const int m = blockIdx.y;
-  if (jh >= JH || m > N) return;
-  const double x = mu[J - JH + jh];
+  if (jh >= ((JH + 7) & ~7)) return;
+  const int R = N + 2 - m;
+  const bool real = jh < JH;
+  const double x = mu[J - JH + (real ? jh : 0)];
   const double s = sqrt((1.0 - x) * (1.0 + x));
   double pmm = 1.0;
   for (int k = 1; k <= m; ++k) pmm *= sqrt((2.0 * k + 1.0) / (2.0 * k)) * s;
-  double *col = P + poff[m] + jh;
+  double *const row = rows && real ? rows + (long long)(m * (N + 2) - m * (m - 1) / 2) * JH + jh : nullptr;
   const double *e = eps + (long long)m * (N + 3);
+  auto put = [&](int r, double v) {
+    const int cnt = (r & 1) ? R / 2 : (R + 1) / 2;
+    blocked[band_at(boff[2 * m + (r & 1)], (cnt + 7) >> 3, r >> 1, jh)] = real ? v : 0.0;
+    if (row && r < R) row[(long long)r * JH] = v;
+  };
   double pm2 = 0.0, pm1 = pmm;
-  col[0] = pmm;
+  put(0, pmm);
   for (int n = m + 1; n <= N + 1; ++n) {
     const double pn = (x * pm1 - e[n - 1] * pm2) / e[n];
-    col[(long long)(n - m) * JH] = pn;
+    put(n - m, pn);
     pm2 = pm1;
     pm1 = pn;
+  }
+  for (int par = 0; par < 2; ++par) {
+    const int cnt = par ? R / 2 : (R + 1) / 2;
+    for (int k = cnt; k < ((cnt + 7) & ~7); ++k) put(2 * k + par, 0.0);
   }
 }
 
@@ -121,11 +137,7 @@ int build_tables(sht_plan *p)
   for (int m = 0; m <= N; ++m)
     for (int n = 0; n <= N + 2; ++n)
       eps[(size_t)m * (N + 3) + n] = (n < m || n == 0) ? 0.0 : std::sqrt(((double)n * n - (double)m * m) / (4.0 * n * n - 1.0));
-  // Legendre table and internal row offsets
-  std::vector<long long> poff(N + 2);
-  long long off = 0;
-  for (int m = 0; m <= N; ++m) { poff[m] = off; off += (long long)(N + 2 - m) * JH; }
-  poff[N + 1] = off;
+  // internal row offsets
   p->h_rowoff.resize(N + 2);
   int ro = 0;
   for (int m = 0; m <= N; ++m) { p->h_rowoff[m] = ro; ro += N + 2 - m; }
@@ -170,21 +182,24 @@ int build_tables(sht_plan *p)
 
   // --- one allocation: the host image's parts, then the device-built tables
   TableArena ar;
-  const size_t o_eps = ar.reserve<double>(eps.size()), o_poff = ar.reserve<long long>(poff.size());
+  const size_t o_eps = ar.reserve<double>(eps.size());
   const size_t o_row = ar.reserve<int>(p->h_rowoff.size()), o_tw = ar.reserve<double2>(NC), o_twI = ar.reserve<double2>(NC);
   const size_t o_rn = ar.reserve<double>(rn.size()), o_tiles = ar.reserve<int2>(tiles.size());
   const size_t o_pairs = ar.reserve<int2>(pairs.size()), o_boff = ar.reserve<long long>(boff.size());
   const size_t o_items = ar.reserve<BandItem>(items.size()), o_rs = ar.reserve<double>((size_t)RS_COUNT * J);
   ar.host_bytes = ar.bytes;
-  const size_t o_mu = ar.reserve<double>(J), o_wgt = ar.reserve<double>(J), o_P = ar.reserve<double>((size_t)off);
+  const size_t o_mu = ar.reserve<double>(J), o_wgt = ar.reserve<double>(J);
+  const bool small = small_supported(p);  // reads row-major rows
+  const size_t o_P = ar.reserve<double>(small ? (size_t)p->R * JH : 0);
   const size_t o_bP = ar.reserve<double>(64 * (size_t)boff.back());
   if ((e = cudaMalloc(&p->d_tables, ar.bytes)) != cudaSuccess) return cuda_fail(e, "cudaMalloc(plan tables)");
   char *const base = static_cast<char *>(p->d_tables);
   auto at = [&](size_t o, auto *&ptr) { ptr = reinterpret_cast<std::remove_reference_t<decltype(ptr)>>(base + o); };
-  at(o_eps, p->d_eps); at(o_poff, p->d_poff); at(o_row, p->d_rowoff); at(o_tw, p->d_tw); at(o_twI, p->d_twI);
+  at(o_eps, p->d_eps); at(o_row, p->d_rowoff); at(o_tw, p->d_tw); at(o_twI, p->d_twI);
   at(o_rn, p->d_rn); at(o_tiles, p->d_spec_tiles); at(o_pairs, p->d_pairs); at(o_boff, p->d_band_off);
-  at(o_items, p->d_band_items); at(o_rs, p->d_rowscale); at(o_mu, p->d_mu); at(o_wgt, p->d_wgt); at(o_P, p->d_P);
+  at(o_items, p->d_band_items); at(o_rs, p->d_rowscale); at(o_mu, p->d_mu); at(o_wgt, p->d_wgt);
   at(o_bP, p->d_band_P);
+  if (small) at(o_P, p->d_P);
 
   // --- Gauss nodes and weights on the device, read back for the row scales
   k_gauss_nodes<<<(J / 2 + 127) / 128, 128, 0, p->stream>>>(J, p->d_mu, p->d_wgt);
@@ -211,17 +226,16 @@ int build_tables(sht_plan *p)
   }
   std::vector<char> image(ar.host_bytes);
   auto put = [&](size_t o, const auto &v) { std::memcpy(image.data() + o, v.data(), sizeof(v[0]) * v.size()); };
-  put(o_eps, eps); put(o_poff, poff); put(o_row, p->h_rowoff); put(o_tw, tw); put(o_twI, twI); put(o_rn, rn);
+  put(o_eps, eps); put(o_row, p->h_rowoff); put(o_tw, tw); put(o_twI, twI); put(o_rn, rn);
   put(o_tiles, tiles); put(o_pairs, pairs); put(o_boff, boff); put(o_items, items); put(o_rs, rs);
   if ((e = cudaMemcpyAsync(base, image.data(), ar.host_bytes, cudaMemcpyHostToDevice, p->stream)) != cudaSuccess)
     return cuda_fail(e, "plan table upload");
 
-  // --- Legendre tables on the device
-  dim3 grid((JH + 127) / 128, N + 1);
-  k_legendre_table<<<grid, 128, 0, p->stream>>>(N, J, JH, p->d_mu, p->d_eps, p->d_poff, p->d_P);
+  // --- Legendre table on the device
+  dim3 grid((JH + 127) / 128, p->M);
+  k_legendre_table<<<grid, 128, 0, p->stream>>>(N, J, JH, p->d_mu, p->d_eps, p->d_band_off, p->d_band_P, p->d_P);
   count_launch();
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "k_legendre_table");
-  if ((rc = build_band_table(p))) return rc;
   if ((e = cudaDeviceGetAttribute(&p->num_sms, cudaDevAttrMultiProcessorCount, p->device)) != cudaSuccess)
     return cuda_fail(e, "SM count");
   if ((e = cudaStreamSynchronize(p->stream)) != cudaSuccess) return cuda_fail(e, "plan tables");
