@@ -1,23 +1,8 @@
-// sht_dmma.cuh -- helpers shared by the FP64 tensor-path Legendre kernels:
-// 16-byte cp.async copies (zero-filling when the source is out of range) and
-// the FP64 mma.sync.m8n8k4 fragment product.
+// sht_dmma.cuh -- the FP64 mma.sync fragment products of the Legendre kernels.
 #pragma once
 
 namespace sht {
 namespace dmma {
-
-__device__ __forceinline__ unsigned smem_u32(const void *p)
-{
-  return static_cast<unsigned>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void cp16(void *dst, const void *src, bool valid)
-{
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(dst)), "l"(src),
-               "r"(valid ? 16 : 0));
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-__device__ __forceinline__ void cp_wait1() { asm volatile("cp.async.wait_group 1;\n" ::); }
-__device__ __forceinline__ void cp_wait0() { asm volatile("cp.async.wait_group 0;\n" ::); }
 
 // d (8x8 FP64 tile, two values per lane) += a (8x4, one per lane) * b (4x8, one per lane)
 __device__ __forceinline__ void mma884(double (&d)[2], double a, double b)
@@ -29,8 +14,11 @@ __device__ __forceinline__ void mma884(double (&d)[2], double a, double b)
       : "d"(a), "d"(b));
 }
 
-// two row tiles and two steps at once: the m8n8k4 products d0 += a0 b0 + a2 b1
-// and d1 += a1 b0 + a3 b1 (rows 0-7 and 8-15 of a 16x8 tile) as one instruction
+// two row tiles and two steps at once: the m8n8k4 products d0 += a0 b0, then
+// a2 b1, and d1 += a1 b0, then a3 b1 (rows 0-7 and 8-15 of a 16x8 tile) as one
+// instruction.  The kernels count on its rounding like the two m8n8k4 steps: a
+// field-level has the same bits whichever of the two its batch's kernel issues
+// (measured on B200, tested on every form the kernels have).
 __device__ __forceinline__ void mma1688(double (&d0)[2], double (&d1)[2], double a0, double a1, double a2, double a3,
                                         double b0, double b1)
 {

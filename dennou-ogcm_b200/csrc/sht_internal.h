@@ -97,7 +97,6 @@ __host__ __device__ inline long long band_at(long long blk, int nrt, int k, int 
 struct sht_plan_s {
   uint32_t magic = 0;
   int I = 0, J = 0, N = 0, K = 0, JH = 0, NC = 0, L = 0;
-  int fa = 0, fb = 0;           // four-step split NC = 2^fa * 2^fb
   long long R = 0;              // internal rows (N+1)(N+4)/2
   double radius = 1.0;
   int device = 0;
@@ -113,7 +112,7 @@ struct sht_plan_s {
   int precision = SHT_PREC_FP64;
   int leg_kernel = 0;  // SHT_OPT_LEGENDRE_KERNEL: 4 single-kernel small-grid transform (plain analysis and synthesis,
                        // im <= 128); the other values all take the band kernels
-  int leg_tile = 0;    // SHT_OPT_LEGENDRE_TILE: kept for the callers that set it, no kernel has a choice of tiles
+  int leg_tile = 0;    // SHT_OPT_LEGENDRE_TILE: kept for the callers that set and read it, selects nothing
 
   // device tables, all in one allocation
   void *d_tables = nullptr;
@@ -227,13 +226,6 @@ bool split_supported(const sht_plan *p);
 // the per-grid FP64 kernels of the time; the band kernels are now the faster on
 // both sides of it (T170, 720: 198 / 209 us against 412 / 324; T341, 960: 1758 /
 // 1792 against 2459 / 2403), so SHT_PREC_FP64 is the mode for speed.
-// --- whole plain transforms of small grids in one kernel (sht_small.cu)
-bool small_supported(const sht_plan *p);
-int launch_small_fwd(const sht_plan *p, const double *g, const double *const *gcol, int ncol, double *w,
-                     double *const *wcol, cudaStream_t s);
-int launch_small_inv(const sht_plan *p, const double *w, const double *const *wcol, int ncol, double *g,
-                     double *const *gcol, cudaStream_t s);
-
 inline bool use_split(const sht_plan *p, bool analysis)
 {
   if (p->precision == SHT_PREC_SPLIT) return true;
@@ -241,6 +233,12 @@ inline bool use_split(const sht_plan *p, bool analysis)
   return (analysis ? p->JH : (p->N + 3) / 2) >= 128;
 }
 
+// --- whole plain transforms of small grids in one kernel (sht_small.cu)
+bool small_supported(const sht_plan *p);
+int launch_small_fwd(const sht_plan *p, const double *g, const double *const *gcol, int ncol, double *w,
+                     double *const *wcol, cudaStream_t s);
+int launch_small_inv(const sht_plan *p, const double *w, const double *const *wcol, int ncol, double *g,
+                     double *const *gcol, cudaStream_t s);
 // plain analysis / synthesis by the single-kernel small-grid transform:
 // chosen with SHT_OPT_LEGENDRE_KERNEL = 4, and by the automatic choice for
 // im = 32 (16 complex points per row), the only size where it measured
@@ -259,7 +257,7 @@ inline int grid_sms(const sht_plan *p)
   return (p->sm_cap > 0 && p->sm_cap < n) ? p->sm_cap : n;
 }
 
-// --- Legendre contraction, split precision on tcgen05 (sht_legendre_tc.cu)
+// --- Legendre contraction, split precision on tcgen05 (sht_legendre_i8.cu)
 int launch_leg_fwd_split(sht_plan *p, const double2 *F, int ncol, double2 *S, cudaStream_t s);
 int launch_leg_inv_split(sht_plan *p, const double2 *S, int ncol, double2 *F, cudaStream_t s);
 void free_split_tables(sht_plan *p);

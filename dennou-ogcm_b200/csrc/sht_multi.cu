@@ -81,14 +81,13 @@ bool live(const sht_multi *m) { return m && m->magic == kMultiMagic; }
 // order) and points each plan at its own stream with the group's Legendre
 // configuration; everything is restored on release.
 struct PlanLease {
-  struct Saved { sht_plan *p; cudaStream_t stream; int precision, leg_kernel, leg_tile, sm_cap; bool timing; };
+  struct Saved { sht_plan *p; cudaStream_t stream; int precision, leg_kernel, sm_cap; bool timing; };
   std::vector<Saved> saved;
   explicit PlanLease(sht_multi *m)
   {
     for (Group &g : m->groups) {
       g.plan->mtx.lock();
-      saved.push_back({g.plan, g.plan->stream, g.plan->precision, g.plan->leg_kernel, g.plan->leg_tile,
-                       g.plan->sm_cap, g.plan->timing.on});
+      saved.push_back({g.plan, g.plan->stream, g.plan->precision, g.plan->leg_kernel, g.plan->sm_cap, g.plan->timing.on});
       g.plan->stream = g.plan->own_stream;
       g.plan->timing.on = false;
       apply(g);
@@ -98,7 +97,6 @@ struct PlanLease {
   {
     g.plan->precision = g.precision;
     g.plan->leg_kernel = g.leg_kernel;
-    g.plan->leg_tile = g.leg_tile;
     g.plan->sm_cap = g.sm_cap;
   }
   ~PlanLease()
@@ -107,7 +105,6 @@ struct PlanLease {
       it->p->stream = it->stream;
       it->p->precision = it->precision;
       it->p->leg_kernel = it->leg_kernel;
-      it->p->leg_tile = it->leg_tile;
       it->p->sm_cap = it->sm_cap;
       it->p->timing.on = it->timing;
       it->p->mtx.unlock();
@@ -184,20 +181,19 @@ int tune_group(Group &g, bool allow_split)
 {
   // the band kernels, the single-kernel transform of small grids, and split
   // precision where allowed
-  struct Cand { int precision, leg_kernel, leg_tile; };
+  struct Cand { int precision, leg_kernel; };
   std::vector<Cand> cands;
-  cands.push_back({SHT_PREC_FP64, 0, 0});
-  if (small_supported(g.plan)) cands.push_back({SHT_PREC_FP64, 4, 0});  // one kernel per direction
+  cands.push_back({SHT_PREC_FP64, 0});
+  if (small_supported(g.plan)) cands.push_back({SHT_PREC_FP64, 4});  // one kernel per direction
   if (allow_split && split_supported(g.plan)) {
-    cands.push_back({SHT_PREC_SPLIT, 0, 0});
-    cands.push_back({SHT_PREC_AUTO, 0, 0});  // split where the contraction is long, FP64 elsewhere
+    cands.push_back({SHT_PREC_SPLIT, 0});
+    cands.push_back({SHT_PREC_AUTO, 0});  // split where the contraction is long, FP64 elsewhere
   }
   float best = 0.f;
   Cand win = cands.front();
   for (const Cand &c : cands) {
     g.precision = c.precision;
     g.leg_kernel = c.leg_kernel;
-    g.leg_tile = c.leg_tile;
     PlanLease::apply(g);
     float ms = 0.f;
     int rc = time_group(g, 3, &ms);
@@ -206,7 +202,7 @@ int tune_group(Group &g, bool allow_split)
   }
   g.precision = win.precision;
   g.leg_kernel = win.leg_kernel;
-  g.leg_tile = win.leg_tile;
+  g.leg_tile = 0;
   g.tuned_ms = best;
   PlanLease::apply(g);
   return SHT_OK;

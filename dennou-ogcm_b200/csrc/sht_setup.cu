@@ -94,14 +94,6 @@ __global__ void k_legendre_table(int N, int J, int JH, const double *__restrict_
   }
 }
 
-static int ilog2_exact(int n)
-{
-  int l = 0;
-  if (n <= 0) return -1;
-  while ((1 << l) < n) ++l;
-  return ((1 << l) == n) ? l : -1;
-}
-
 namespace {
 
 // The plan's tables share one device allocation: parts are reserved first,
@@ -124,9 +116,6 @@ struct TableArena {
 int build_tables(sht_plan *p)
 {
   const int I = p->I, J = p->J, N = p->N, JH = p->JH, NC = p->NC;
-  int lg = p->zonal ? 0 : ilog2_exact(NC);
-  p->fb = lg / 2;
-  p->fa = lg - p->fb;
   p->R = (long long)(N + 1) * (N + 4) / 2;
   p->M = p->zonal ? 1 : N + 1;
   p->L = p->zonal ? N + 1 : (N + 1) * (N + 1);

@@ -7,8 +7,8 @@
 //   smem desc: [0,14) start >> 4, [16,30) leading-dim byte offset >> 4,
 //              [32,46) stride-dim byte offset >> 4, [46,48) version = 1,
 //              [49,52) base offset, [52] lbo mode, [61,64) swizzle (0 = none)
-//   instr desc (kind::f16): [4,6) D format (1 = F32), [7,10) A format
-//              (1 = BF16), [10,13) B format, [15] A major, [16] B major
+//   instr desc (kind::i8): [4,6) D format (2 = S32), [7,10) A format
+//              (1 = signed 8-bit), [10,13) B format, [15] A major, [16] B major
 //              (0 = K-major), [17,23) N >> 3, [24,29) M >> 4.
 // K-major operands without swizzle use the interleaved canonical layout:
 // core matrices of 8 rows x 16 bytes (rows 16 B apart).  Here the two core
@@ -34,12 +34,6 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo_bytes
   d |= (uint64_t)((sbo_bytes >> 4) & 0x3FFFu) << 32;
   d |= (uint64_t)1u << 46;  // version
   return d;                 // base offset 0, lbo mode 0, no swizzle
-}
-
-// BF16 x BF16 -> F32, both operands K-major.
-__host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N)
-{
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
 // signed 8-bit x signed 8-bit -> S32 (kind::i8), both operands K-major:
@@ -70,16 +64,6 @@ __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.
 // generic-proxy global stores of this thread made visible to later bulk copies
 __device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;\n" ::: "memory"); }
 
-// D[tmem] (+)= A[smem] * B[smem]^T, issued by one thread
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate)
-{
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
-}
-
 // D[tmem] (+)= A[smem] * B[smem]^T with 8-bit integer operands and exact
 // 32-bit integer accumulation, issued by one thread
 __device__ __forceinline__ void mma_s8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate)
@@ -97,22 +81,6 @@ __device__ __forceinline__ void mma_commit(uint64_t *mbar)
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_addr(mbar)));
 }
 
-// 32 lanes x 32 bits, 16 consecutive columns -> 16 registers per thread
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16])
-{
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-}
-// 32 lanes x 32 bits, 8 consecutive columns -> 8 registers per thread
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8])
-{
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "r"(taddr));
-}
 // 32 lanes x 32 bits, 4 consecutive columns -> 4 registers per thread
 __device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&r)[4])
 {

@@ -438,7 +438,8 @@ SHT_API int sht_multi_synchronize(sht_multi *multi);
 SHT_API int sht_multi_groups(const sht_multi *multi, int *ngroups);
 SHT_API int sht_multi_group_info(const sht_multi *multi, int group, int *ncol, int *precision,
                                  int *legendre_kernel, float *tuned_ms);
-/* The SHT_OPT_LEGENDRE_TILE value the group runs with (the tuner's choice). */
+/* The SHT_OPT_LEGENDRE_TILE value of the group: the plan's, or 0 where the tuner
+ * chose (it selects nothing). */
 SHT_API int sht_multi_group_tile(const sht_multi *multi, int group, int *legendre_tile);
 /* SMs the group's persistent kernels size their grids for, so that the
  * groups run side by side (0: the whole GPU).  With autotuning the build
