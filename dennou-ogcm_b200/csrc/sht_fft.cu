@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(256) k_zonal_inv(FftArgs a)
 
 // Longitude counts with a prime factor above 5 (or without a product of two
 // radices up to 32, e.g. 1944; counts with factors 3 and 5 otherwise take the
-// kernels of sht_fft_mixed.cu, 17-29 times faster on the T106 grid): the
+// kernels of sht_fft_mixed.cu, 21 and 34 times faster on the T106 grid): the
 // transform by direct summation, G^m = s_j sum_i q_i e^{-2 pi i m i / I} for m <= N and its
 // inverse, with e^{-2 pi i t / I} = twI[t] for t < I/2 and -twI[t - I/2]
 // otherwise.  A block handles four mirrored row pairs of one field-level

@@ -22,7 +22,8 @@
 // blocks per SM).  What it replaces, the direct sum over longitudes, is O(I N)
 // per row and bound by its FP64 products.  The T106 grid (320 x 160, 180
 // field-levels, 123 MB per direction): forward / inverse 0.730 / 1.289 ms ->
-// 0.031 / 0.037 ms, 4.0 / 3.3 TB/s; 192 x 96, 74 columns: 61 / 112 -> 6.9 / 7.1 us.
+// 0.034 / 0.038 ms with cold caches, 3.6 / 3.2 TB/s (0.031 / 0.037 back to back);
+// 192 x 96, 74 columns: 61 / 112 -> 9.5 / 11.3 us (6.9 / 7.1 back to back).
 #include "sht_fft_tile.cuh"
 #include "sht_fft_mixed.cuh"
 
@@ -697,7 +698,8 @@ struct MixShape {
 };
 
 // Pairs in the inverse up to radix 20; otherwise rows of I/2 while their
-// radices stay at 16, then pairs.  Measured, rows / pairs, us: inverse im = 96,
+// radices stay at 16, then pairs.  Stage times (each with a launch gap of a few
+// us), rows / pairs, us: inverse im = 96,
 // 2000 field-levels 52 / 39, 240, 300 56 / 37, 320, 180 48 / 41, 480, 80 50 /
 // 62, 640, 60 125 / 72; forward 96 40 / 39, 192, 500 36 / 39, 320 38 / 42, 480
 // 39 / 67, 640 86 / 76.

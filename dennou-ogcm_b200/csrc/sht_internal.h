@@ -224,8 +224,9 @@ bool split_supported(const sht_plan *p);
 // the analysis, (nm+3)/2 degrees of one parity in the synthesis).  That is the
 // mode's documented meaning.  The line was drawn where the int8 digit kernel beat
 // the per-grid FP64 kernels of the time; the band kernels are now the faster on
-// both sides of it (T170, 720: 198 / 209 us against 412 / 324; T341, 960: 1758 /
-// 1792 against 2459 / 2403), so SHT_PREC_FP64 is the mode for speed.
+// both sides of it (synthesis / analysis, T170, 720: 195 / 208 us against 403 /
+// 327; T341, 960: 1746 / 1832 against 2439 / 2384), so SHT_PREC_FP64 is the mode
+// for speed.
 inline bool use_split(const sht_plan *p, bool analysis)
 {
   if (p->precision == SHT_PREC_SPLIT) return true;
@@ -242,8 +243,8 @@ int launch_small_inv(const sht_plan *p, const double *w, const double *const *wc
 // plain analysis / synthesis by the single-kernel small-grid transform:
 // chosen with SHT_OPT_LEGENDRE_KERNEL = 4, and by the automatic choice for
 // im = 32 (16 complex points per row), the only size where it measured
-// faster than the batched kernels (T10, 480 field-levels: round trip 26
-// against 37 us); in FP64 only (split precision keeps the batched path)
+// faster than the batched kernels (T10, 480 field-levels: round trip 23
+// against 25 us); in FP64 only (split precision keeps the batched path)
 inline bool wants_small(const sht_plan *p) { return p->leg_kernel == 4 || (p->leg_kernel == 0 && p->NC == 16); }
 inline bool use_small(const sht_plan *p, bool analysis)
 {

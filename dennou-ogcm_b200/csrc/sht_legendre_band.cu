@@ -7,9 +7,9 @@
 //   synthesis (:212-216):
 //     F[m][col][par JH + jh] = sum over the r of parity par of Pbar S[row][col].
 //
-// Each is a dense product per (m, par) on the FP64 tensor path
-// (mma.sync.m8n8k4.f64; 37 TF/s is also the FMA pipe's rate, the two share
-// it).  A block takes one work item -- up to TM 8-row tiles of the output
+// Each is a dense product per (m, par) on the FP64 tensor path (mma.sync f64:
+// m16n8k8 for pairs of 8-row tiles, m8n8k4 for an odd tile and for tails of up to
+// four terms; 37 TF/s is also the FMA pipe's rate, the two share it).  A block takes one work item -- up to TM 8-row tiles of the output
 // (degrees of one parity in the analysis, latitudes in the synthesis) -- and
 // 8 CW field-level columns.  Warp w owns 8 columns (real and imaginary parts
 // are two 8-wide tiles) and every RW-th row tile, CW RW = W, so a warp's
@@ -44,8 +44,8 @@
 // to 8-row tiles counted; the inner loop alone reaches 97 %), the Fourier
 // array's traffic and the units' latency below.  Measured against the kernels it
 // replaced (analysis / synthesis, us): T42, 3095 field-levels 52 / 48 -> 37 /
-// 35; T85, 480: 39.6 / 42.0 -> 30.7 / 30.7; 320 x 160 (T106), 180: 70 / 82 -> 27
-// / 25; T170, 720: 434 / 396 -> 207 / 195; T341, 240: 909 / 987 -> 483 / 475
+// 35; T85, 480: 39.6 / 42.0 -> 31.5 / 30.7; 320 x 160 (T106), 180: 70 / 82 -> 25
+// / 26; T170, 720: 434 / 396 -> 208 / 195; T341, 240: 909 / 987 -> 483 / 473
 // (30.5 TF/s of the 37 executed).  Filling the stages with cp.async from the
 // consumer warps instead took 268 / 264 us at T170: their copy instructions
 // (up to ten per product) held the pipe at 61 %.
@@ -473,7 +473,7 @@ int even_split(int tiles, int cap)
 
 // 8 tiles of accumulators are what 128 registers hold; items of up to 11 (160
 // registers, two teams) re-read the data less often but took 506 / 508 us at
-// T341 where these take 483 / 475.
+// T341 where these take 483 / 473.
 constexpr int kItemCap = 8;
 
 }  // namespace
@@ -699,9 +699,9 @@ int launch_band(const sht_plan *p, BandArgs a, cudaStream_t s)
   const int tm = INV ? p->band_ti : p->band_tf;
   // One block of three teams, or three blocks of one.  The teams share the SM's
   // units, which pays where a unit is long (analysis / synthesis, T170, 720:
-  // 221 / 215 -> 209 / 197 us, T341, 240: 506 / 508 -> 483 / 475); below, blocks
-  // that start and end apart are level or ahead (T85, 480: 32.8 / 30.7 either way,
-  // T42, 3095: 39.8 / 36.9 shared, 36.9 / 34.8 apart).
+  // 221 / 215 -> 208 / 195 us, T341, 240: 506 / 508 -> 483 / 473); below, blocks
+  // that start and end apart are level or ahead (T85, 480: 31.5 / 30.7 either way,
+  // T42, 3095: 39.8 / 36.9 shared, 37 / 35 apart).
   if (p->N > 127) return run_band<4, 8, 4, 3, 1, INV>(p, a, s);
   if (tm <= 6) return run_band<4, 6, 4, 1, 3, INV>(p, a, s);
   return run_band<4, 8, 4, 1, 3, INV>(p, a, s);

@@ -24,7 +24,7 @@
 // for m > 0, SpmlUtil's wa layout) as the batched path.
 //
 // It is faster than the batched path only for the smallest grids (480
-// field-levels, round trip: T10 26 against 37 us, T21 45 against 28): each block re-reads the Legendre
+// field-levels, round trip: T10 23 against 25 us, T21 45 against 29): each block re-reads the Legendre
 // table for its two levels, where the batched kernels use every table row on
 // 32 columns, and its phases (loads, transform, contraction, stores) run
 // one after the other in blocks that the shared-memory arrays keep few per SM.
