@@ -452,8 +452,10 @@ SHT_API int sht_multi_destroy(sht_multi *multi);
 /* ------------------------------------------------------------ diagnostics */
 
 /* Device time in milliseconds of the kernels of the last *_dev call, summed
- * per stage (fft, legendre, spectral); NULL entries are skipped.  Timing is
- * recorded only when enabled with sht_set_timing(plan, 1). */
+ * per stage (fft, legendre, spectral); NULL entries are skipped.  A kernel that
+ * does several stages counts as one: contraction and layout conversion of a few
+ * field-levels as legendre, the single-kernel small-grid transform as fft.
+ * Timing is recorded only when enabled with sht_set_timing(plan, 1). */
 SHT_API int sht_set_timing(sht_plan *plan, int on);
 SHT_API int sht_last_timing(const sht_plan *plan, float *ms_fft, float *ms_legendre,
                     float *ms_spectral);
